@@ -297,8 +297,8 @@ extern "C" int vk_create(const vk_network *net, int max_cols, int max_layers, in
     TRY(dalloc(h, &h->d_col_end, max_cols));
     TRY(dalloc(h, &h->d_cols, max_cols));
     TRY(dalloc(h, &h->d_order, max_cols));
-    TRY(dalloc(h, &h->d_queue, 1));
-    TRY(dalloc(h, &h->d_queue2, 1));
+    TRY(dalloc(h, &h->d_queue, 1 + max_cols));
+    TRY(dalloc(h, &h->d_queue2, 1 + max_cols));
     TRY(cudaStreamCreateWithFlags(&h->stream2, cudaStreamNonBlocking) == cudaSuccess
             ? VK_OK : fail(h, VK_ECUDA, "cudaStreamCreate (FP64 branch)"));
     TRY(cudaEventCreateWithFlags(&h->ev_fork, cudaEventDisableTiming) == cudaSuccess
@@ -602,6 +602,20 @@ static void ensure_geometry(vk_handle *h, int flags) {
     h->geo_flags = flags;
 }
 
+// Kernels of one attempt: rates, stage and the FP64 branch's six -- in mixed
+// mode two such branches beside the routing and the mixed branch's five.
+static int attempt_launches(const vk_handle *h) { return h->precision == VK_PREC_MIXED ? 20 : 8; }
+
+// k1, yk2, the second right-hand side and k2 from the FP64 factors.
+static void enqueue_solves64(vk_handle *h, const DevNet &net, const DevBatch &b, int flags, cudaStream_t s) {
+    vk::Work &w = h->w;
+    vk::launch_fwd64(net, b, w.G, w.dB, w.dC, w.f, w.z, w.status, s);
+    vk::launch_back64(net, b, w.G, w.dB, w.dC, w.z, w.k1, w.y, w.yk2, w.status, s);
+    vk::launch_rates(net, b, w.yk2, w.f, nullptr, nullptr, nullptr, nullptr, w.k1, w.dt, w.geo, flags, false, s);
+    vk::launch_fwd64(net, b, w.G, w.dB, w.dC, w.f, w.z, w.status, s);
+    vk::launch_back64(net, b, w.G, w.dB, w.dC, w.z, w.k2, w.y, nullptr, w.status, s);
+}
+
 // Enqueue the kernels of one Ros2 attempt for the columns b.active selects
 // (all when NULL): device state in, w.sol / w.ymix_out / w.delta out.
 static void enqueue_attempt_kernels(vk_handle *h, const DevNet &net, const DevBatch &b, int flags,
@@ -612,12 +626,9 @@ static void enqueue_attempt_kernels(vk_handle *h, const DevNet &net, const DevBa
     vk::launch_rates(net, b, w.y, w.f, w.jv, w.dA, w.dB, w.dC, nullptr, w.dt, w.geo, flags, true, s);
     if (timed) cudaEventRecord(h->ev[1], s);
     if (h->precision == VK_PREC_FP64) {
-        vk::launch_lu_fwd_f64(net, b, w, w.f, w.z, flags, s);
+        vk::launch_lu64(net, b, w, s);
         if (timed) cudaEventRecord(h->ev[2], s);
-        vk::launch_back_f64(net, b, w.G, w.dB, w.z, w.k1, w.y, w.yk2, w.status, s);
-        vk::launch_rates(net, b, w.yk2, w.f, nullptr, nullptr, nullptr, nullptr, w.k1, w.dt, w.geo, flags, false, s);
-        vk::launch_solve_f64(net, b, w.G, w.dB, w.dC, w.f, w.z, w.k2, w.status, s);
-        h->launches += 6;
+        enqueue_solves64(h, net, b, flags, s);
     } else {
         // route: fallback[c] = column goes to FP64 this attempt, act32[c] = mixed
         cudaMemsetAsync(w.sweeps, 0, sizeof(int), s);
@@ -632,10 +643,8 @@ static void enqueue_attempt_kernels(vk_handle *h, const DevNet &net, const DevBa
         DevBatch br = b;
         br.active = w.routed;
         br.queue = h->d_queue2;
-        vk::launch_lu_fwd_f64(net, br, w, w.f, w.z, flags, s2);
-        vk::launch_back_f64(net, br, w.G, w.dB, w.z, w.k1, w.y, w.yk2, w.status, s2);
-        vk::launch_rates(net, br, w.yk2, w.f, nullptr, nullptr, nullptr, nullptr, w.k1, w.dt, w.geo, flags, false, s2);
-        vk::launch_solve_f64(net, br, w.G, w.dB, w.dC, w.f, w.z, w.k2, w.status, s2);
+        vk::launch_lu64(net, br, w, s2);
+        enqueue_solves64(h, net, br, flags, s2);
         cudaEventRecord(h->ev_join, s2);
         DevBatch b32 = b;
         b32.active = w.act32;
@@ -649,15 +658,13 @@ static void enqueue_attempt_kernels(vk_handle *h, const DevNet &net, const DevBa
         // is still in place: neither branch wrote it)
         DevBatch bf = b;
         bf.active = w.failed;
-        vk::launch_lu_fwd_f64(net, bf, w, w.f, w.z, flags, s);
-        vk::launch_back_f64(net, bf, w.G, w.dB, w.z, w.k1, w.y, w.yk2, w.status, s);
-        vk::launch_rates(net, bf, w.yk2, w.f, nullptr, nullptr, nullptr, nullptr, w.k1, w.dt, w.geo, flags, false, s);
-        vk::launch_solve_f64(net, bf, w.G, w.dB, w.dC, w.f, w.z, w.k2, w.status, s);
-        h->launches += 16;
+        vk::launch_lu64(net, bf, w, s);
+        enqueue_solves64(h, net, bf, flags, s);
     }
     if (timed) cudaEventRecord(h->ev[3], s);
     vk::launch_stage(net, b, w, flags, mtol, atol, s);
     if (timed) cudaEventRecord(h->ev[4], s);
+    h->launches += attempt_launches(h);
 }
 
 static int enqueue_attempt(vk_handle *h, int flags, bool timed) {
@@ -1217,7 +1224,7 @@ static void run_body(vk_handle *h, const vk::RunCtrl &cc, int ga) {
 
 // Launches of one replay of h's body (the gpu_launches count).
 static int body_launches(const vk_handle *h, int ga) {
-    return ga * (h->precision == VK_PREC_MIXED ? 17 : 7) + 1;
+    return ga * (attempt_launches(h) + 1) + 1;
 }
 
 // A column that stopped with an error status fails the call.

@@ -114,7 +114,8 @@ struct DevBatch {
     const double *spf;         // [ncols][VK_SP_NF][ni]
     const int *active;         // [ncols] non-zero = column takes part (NULL = all)
     const int *order;          // [ncols] columns by decreasing nz (work-queue order)
-    unsigned *queue;           // [1] next queue position (zeroed before each launch)
+    unsigned *queue;           // [1 + ncols] next queue position, then per column how many of
+                               //  its halves are done (zeroed before each launch)
     int nsm;                   // SMs of the device
     int cps;                   // resident CTAs per SM of the per-column kernels
                                // (0: each kernel's own default)
@@ -237,14 +238,13 @@ void launch_rates(const DevNet &net, const DevBatch &b, const double *y, double 
                   double *jv, double *dA, double *dB, double *dC, const double *k1,
                   const double *dt, const double *geo, int flags, bool with_jac, cudaStream_t s);
 void launch_geometry(const DevNet &net, const DevBatch &b, double *geo, int flags, cudaStream_t s);
-void launch_lu_fwd_f64(const DevNet &net, const DevBatch &b, const Work &w,
-                       const double *rhs, double *z, int flags, cudaStream_t s);
-void launch_back_f64(const DevNet &net, const DevBatch &b, const double *G,
-                     const double *dB, const double *z, double *x,
-                     const double *y, double *yk2, int *status, cudaStream_t s);
-void launch_solve_f64(const DevNet &net, const DevBatch &b, const double *G,
-                      const double *dB, const double *dC, const double *rhs,
-                      double *zbuf, double *x, int *status, cudaStream_t s);
+cudaError_t init_lu64(int n);
+void launch_lu64(const DevNet &net, const DevBatch &b, const Work &w, cudaStream_t s);
+void launch_fwd64(const DevNet &net, const DevBatch &b, const double *G, const double *dB,
+                  const double *dC, const double *rhs, double *z, int *status, cudaStream_t s);
+void launch_back64(const DevNet &net, const DevBatch &b, const double *G, const double *dB,
+                   const double *dC, double *z, double *x, const double *y, double *yk2, int *status,
+                   cudaStream_t s);
 void launch_stage(const DevNet &net, const DevBatch &b, const Work &w, int flags,
                   double mtol, double atol, cudaStream_t s);
 void launch_refine(const DevNet &net, const DevBatch &b, const Work &w, const double *rhs,
