@@ -979,7 +979,7 @@ extern "C" int vk_photo_setup(vk_handle *h, int nbins, const double *bins, const
     if (!rc) rc = upload(h, &dki, kiv);
     double **big[] = {&p.tau, &p.dflux_u, &p.dflux_d};
     for (double **q : big) if (!rc) rc = dalloc(h, q, st);
-    double **lay[] = {&p.w0, &p.aflux, &p.aflux_prev};
+    double **lay[] = {&p.w0, &p.aflux, &p.aflux_prev, &p.cX, &p.cD, &p.cU};
     for (double **q : lay) if (!rc) rc = dalloc(h, q, ly);
     if (!rc) rc = dalloc(h, &p.J, (size_t)h->max_layers * nch);
     if (!rc) rc = dalloc(h, &h->d_phmask, h->max_cols);

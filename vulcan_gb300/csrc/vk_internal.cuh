@@ -188,6 +188,7 @@ struct PhotoDev {
     double sl_angle, edd, f_diurnal, flux_atol;
     double *tau, *dflux_u, *dflux_d;   // [(L + ncols)][nbins] staggered
     double *w0, *aflux, *aflux_prev;   // [L][nbins]
+    double *cX, *cD, *cU;      // [L][nbins] two-stream coefficients of the current update
     double *J;                 // [L][nch]
     // temperature-dependent cross sections (vk_photo_set_cross_T); NULL: none
     const int *abs_tslot;      // [nabs] row of cross_T, or -1
