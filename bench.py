@@ -6,8 +6,8 @@ slots), nz ~ U{60..200} (sum 66 752 layers), T/Kzz/metallicity/C-O seeded
 (vulcan_gb300.configs.config2_columns, seed 2).  One bench step = one Ros2 step
 (attempts until accepted, device step control) of every column.
 
-value  = accepted column-steps per second of the mixed path (FP32 tensor-core
-         block LU + FP64 refinement) with the state resident in HBM, over the
+value  = accepted column-steps per second of the mixed path (FP32 block LU +
+         FP64 refinement) with the state resident in HBM, over the
          timed steps after the warm-up (early steps from const_mix).
 e2e    = the same through the C-ABI with host buffers: every step copies the
          state (y, ymix) host->device, runs one step, and copies y back.
@@ -61,17 +61,6 @@ def peaks():
         d = json.load(open(p))
         return d.get('hbm_gbs', 6800.0), 'measured'
     return 6800.0, 'fallback'
-
-
-def tf32_peak():
-    """Dense TF32 tensor rate: half the measured dense BF16 burst rate (the
-    same tensor cores at half the BF16 throughput), else the fallback."""
-    p = os.path.join(REPO, 'MEASURED_PEAKS.json')
-    if os.path.exists(p):
-        d = json.load(open(p))
-        if 'bf16_tflops' in d:
-            return d['bf16_tflops'] / 2, 'measured bf16 burst / 2 (TF32 dense)'
-    return 1900.0 / 2, 'fallback bf16 / 2 (TF32 dense)'
 
 
 # ------------------------------------------------------------ CPU baseline
@@ -401,15 +390,8 @@ def run_gpu(args):
     if dom == 'lu':
         fl = float(L) * ni ** 3 * 2.0          # Gauss-Jordan: ni^3 FMA per layer
         ach = fl / (am['lu'] * 1e-3) / 1e12
-        if ni <= 128:                          # the tensor-core factorisation (default)
-            ptf, src = tf32_peak()
-            roof = {'bound': 'tensor', 'kernel': 'k_lu_tc (+k_prep32)', 'achieved': ach, 'peak': ptf,
-                    'unit': 'TFLOP/s', 'peak_source': src,
-                    'fp32_core': {'peak': round(peak32, 3), 'frac': round(ach / peak32, 4),
-                                  'peak_source': 'measured cuBLAS SGEMM 8192^3 (no TF32) in this run'}}
-        else:
-            roof = {'bound': 'fp32', 'kernel': 'k_lu32 (+k_prep32)', 'achieved': ach, 'peak': peak32,
-                    'unit': 'TFLOP/s', 'peak_source': 'measured cuBLAS SGEMM 8192^3 (no TF32) in this run'}
+        roof = {'bound': 'fp32', 'kernel': 'k_lu32 (+k_prep32)', 'achieved': ach, 'peak': peak32,
+                'unit': 'TFLOP/s', 'peak_source': 'measured cuBLAS SGEMM 8192^3 (no TF32) in this run'}
     else:
         # refinement + second RHS: every sweep streams the FP32 inverses twice
         by = float(L) * stride * 4 * 2 * 2 * 3

@@ -296,17 +296,14 @@ VK_API int  vk_compute_k(vk_handle *h);
  * The per-column kernels take columns from a work queue; their grid is
  * ctas_per_sm x SMs CTAs.  kernel: VK_TUNE_*; ctas_per_sm 0..8 (0: the
  * kernel's built-in default, or VK_CTAS_PER_SM from the environment);
- * variant: for VK_TUNE_LU32 the register tiling of the FP32 Gauss-Jordan,
- * 0..3 covering blocks up to 48, 80, 112, 160 species, 4: the tensor-core
- * factorisation (tcgen05, blocks up to 128 species) with one warp eliminating
- * each 16-pivot panel, or 5: the same with the four warps of its CTA
- * eliminating the panel together (identical factors) (-1: the default for
- * ni, variant 5 up to 128 species; a variant smaller than ni is refused),
- * ignored otherwise.
+ * variant: for VK_TUNE_LU32 the register tiling of the FP32 Gauss-Jordan:
+ * 0..3 at least the one for blocks of 48, 80, 112, 160 species, 4 and 5 (up
+ * to 128 species) and -1 the smallest that holds ni; a variant smaller than
+ * ni is refused.  Every variant gives the same factors.  Ignored otherwise.
  * A change drops the captured vk_run graph, which is captured again. */
 #define VK_TUNE_LU32    0   /* k_lu32: FP32 block-Thomas factorisation        */
-#define VK_TUNE_LU64    1   /* k_lu_fwd_f64: FP64 factorisation + first sweep */
-#define VK_TUNE_SWEEP64 2   /* k_back_f64, k_solve_f64: FP64 sweeps           */
+#define VK_TUNE_LU64    1   /* k_lu64: FP64 factorisation                    */
+#define VK_TUNE_SWEEP64 2   /* k_sweep64: FP64 sweeps                         */
 #define VK_TUNE_REFINE  3   /* k_refine: FP64 refinement with FP32 factors    */
 #define VK_TUNE_N       4
 VK_API int  vk_set_launch(vk_handle *h, int kernel, int ctas_per_sm, int variant);

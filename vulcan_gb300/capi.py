@@ -16,8 +16,8 @@ VK_PREC_FP64, VK_PREC_MIXED = 0, 1
 VK_F_MOLDIFF, VK_F_TOPFLUX, VK_F_BOTFLUX = 1, 2, 4
 VK_TUNE_LU32, VK_TUNE_LU64, VK_TUNE_SWEEP64, VK_TUNE_REFINE = 0, 1, 2, 3
 LU32_TILING_CAP = (48, 80, 112, 160, 128, 128)  # species each LU32 variant covers
-LU32_TC = 4                                # the tensor-core factorisation (k_lu_tc)
-LU32_TC_COOP = 5                           # the same, four warps per panel
+LU32_TC = 4                                # the smallest register tiling that holds the block
+LU32_TC_COOP = 5                           # the same (kept for callers that name it)
 (ATM_M, ATM_N0, ATM_TCO, ATM_G, ATM_DZI, ATM_KZZ, ATM_VZ, ATM_TI, ATM_HPI, ATM_HP,
  ATM_PICO, ATM_PICOU, ATM_DZ) = range(13)
 ATM_NF = 13

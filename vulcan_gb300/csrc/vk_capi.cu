@@ -29,7 +29,6 @@ struct vk_handle {
     double refine_tol = 1e-10;
     double route_dt0 = INFINITY;  // vk_set_route: FP64 from this step size until a failure lowers it
     int geo_flags = -1;         // flags the transport geometry was built for (-1: stale)
-    CUtensorMap tmap_d32{};     // k_lu_tc's view of w.D32 (mixed mode, ni <= 128)
     int ncols = 0, L = 0;
     std::vector<int> col_off, col_end;  // first / one past last layer of each column
     int slot_cap = 0;                   // > 0: slotted layout (vk_set_columns_slotted)
@@ -46,6 +45,9 @@ struct vk_handle {
     int *d_jpos = nullptr;
     int *d_jrow = nullptr, *d_jcol = nullptr, *d_jrowptr = nullptr, *d_jmap = nullptr;
     double *d_compo = nullptr;
+    int npc = 0;                        // pieces of the Jacobian rows (k_refine)
+    int2 *d_pc = nullptr;
+    int *d_rpcptr = nullptr, *d_rpc = nullptr;
     int nxm = 0, nh = 0;                // extra source products, derivative half terms
     int *d_porder = nullptr, *d_src_slot = nullptr, *d_xmul_pair = nullptr;
     double *d_src_c = nullptr, *d_xmul_fac = nullptr, *d_hjcoef = nullptr;
@@ -73,7 +75,7 @@ struct vk_handle {
     int nsm = 0;                        // SMs of the device
     int cps = 0;                        // VK_CTAS_PER_SM override (0: kernel defaults)
     int cps_k[VK_TUNE_N] = {0, 0, 0, 0}; // vk_set_launch: CTAs per SM per kernel
-    int lu32_tiling = -1;               // vk_set_launch: k_lu32 tiling (-1: by ni)
+    int lu32_tiling = -1;               // vk_set_launch: k_lu32 variant (-1: by ni)
     int occ_rates = 0, occ_prep = 0;    // resident CTAs per SM of k_rates / k_prep32
     double *d_k = nullptr, *d_atm = nullptr, *d_Dzz = nullptr, *d_spf = nullptr;
     vk::Work w{};
@@ -99,6 +101,7 @@ struct vk_handle {
         n.src_nu = d_src_nu; n.jterm_nu = d_jterm_nu;
         n.jptr = d_jptr; n.jterm = d_jterm; n.jpos = d_jpos; n.compo = d_compo;
         n.jrow = d_jrow; n.jcol = d_jcol; n.jrowptr = d_jrowptr; n.jmap = d_jmap;
+        n.npc = npc; n.pc = d_pc; n.rpcptr = d_rpcptr; n.rpc = d_rpc;
         n.nxm = nxm; n.nh = nh; n.porder = d_porder; n.src_slot = d_src_slot; n.src_c = d_src_c;
         n.xmul_pair = d_xmul_pair; n.xmul_fac = d_xmul_fac; n.hk = d_hk; n.hptr = d_hptr;
         n.hfac = d_hfac; n.hjterm = d_hjterm; n.hjptr = d_hjptr; n.hjcoef = d_hjcoef;
@@ -195,28 +198,18 @@ extern "C" void vk_destroy(vk_handle *h) {
     delete h;
 }
 
-// Buffers of the mixed-precision path: the FP32 inverses (packed n x n per
-// layer) and the scaled blocks, sized for k_lu32's packed layout or k_lu_tc's
-// zero-padded NP x NP tiles, with the tensor map k_lu_tc loads them through.
+// Buffers of the mixed-precision path: the FP32 inverses and the scaled blocks
+// (packed n x n per layer, 16-byte aligned) and the refinement's vectors.
 static int alloc_mixed(vk_handle *h) {
     const size_t st = (size_t)((h->ni * h->ni + 3) & ~3);
-    const bool tc = vk::lu_tc_supported(h->ni);
-    const size_t sd = tc ? std::max(st, vk::lu_tc_block_floats(h->ni)) : st;
     const size_t lv = (size_t)h->max_layers * h->ni;
     int rc = dalloc(h, &h->w.G32, (size_t)h->max_layers * st);
-    if (!rc) rc = dalloc(h, &h->w.D32, (size_t)h->max_layers * sd);
+    if (!rc) rc = dalloc(h, &h->w.D32, (size_t)h->max_layers * st);
     if (!rc) rc = dalloc(h, &h->w.wcf, lv);
     if (!rc) rc = dalloc(h, &h->w.wcb, lv);
     if (!rc) rc = dalloc(h, &h->w.raf, lv);
     if (!rc) rc = dalloc(h, &h->w.xf, lv);
-    if (rc) return rc;
-    if (tc) {
-        cudaError_t e = vk::lu_tc_make_map(&h->tmap_d32, h->w.D32, h->ni, h->max_layers);
-        if (e != cudaSuccess)
-            return fail(h, VK_ECUDA, std::string("tensor map of the scaled blocks: ") + cudaGetErrorString(e));
-        h->w.tmap_d32 = &h->tmap_d32;
-    }
-    return VK_OK;
+    return rc;
 }
 
 extern "C" int vk_create(const vk_network *net, int max_cols, int max_layers, int precision,
@@ -279,6 +272,34 @@ extern "C" int vk_create(const vk_network *net, int max_cols, int max_layers, in
     TRY(upload(h, &h->d_jcol, net->jcol));
     TRY(upload(h, &h->d_jrowptr, net->jrowptr));
     TRY(upload(h, &h->d_jmap, net->jmap));
+    {
+        // rows cut into pieces of at most `lim` entries, longest first: a warp's
+        // 32 pieces then have similar lengths (an uncut row of an abundant species
+        // holds 31 other lanes for its whole length)
+        const int lim = h->ni <= 128 ? 24 : 128;
+        std::vector<int2> pc;
+        std::vector<int> row;
+        for (int r = 0; r < h->ni; ++r) {
+            const int a = net->jrowptr[r], len = net->jrowptr[r + 1] - a, k = (len + lim - 1) / lim;
+            for (int i = 0; i < k; ++i) {
+                const int x0 = len * i / k, x1 = len * (i + 1) / k;
+                pc.push_back(make_int2(a + x0, x1 - x0));
+                row.push_back(r);
+            }
+        }
+        std::vector<int> ord(pc.size()), rp(h->ni + 1, 0), rl(pc.size());
+        for (size_t i = 0; i < ord.size(); ++i) ord[i] = (int)i;
+        std::stable_sort(ord.begin(), ord.end(), [&](int a, int c2) { return pc[a].y > pc[c2].y; });
+        std::vector<int2> sorted(pc.size());
+        std::vector<int> at(pc.size());
+        for (size_t i = 0; i < ord.size(); ++i) { sorted[i] = pc[ord[i]]; at[ord[i]] = (int)i; }
+        for (size_t i = 0; i < pc.size(); ++i) { rp[row[i] + 1] = (int)i + 1; rl[i] = at[i]; }
+        for (int r = 0; r < h->ni; ++r) rp[r + 1] = std::max(rp[r + 1], rp[r]);
+        h->npc = (int)pc.size();
+        TRY(upload(h, &h->d_pc, sorted));
+        TRY(upload(h, &h->d_rpcptr, rp));
+        TRY(upload(h, &h->d_rpc, rl));
+    }
     h->nxm = (int)net->xmul_pair.size();
     h->nh = (int)net->hk.size();
     TRY(upload(h, &h->d_porder, net->porder));
@@ -321,7 +342,7 @@ extern "C" int vk_create(const vk_network *net, int max_cols, int max_layers, in
     TRY(dalloc(h, &h->d_spf, (size_t)max_cols * VK_SP_NF * ni));
     vk::Work &w = h->w;
     double **vecs[] = {&w.y, &w.ymix, &w.yk2, &w.f, &w.k1, &w.k2, &w.z, &w.sol, &w.ymix_out,
-                       &w.dA, &w.dB, &w.dC, &w.r, &w.f2, &w.rs, &w.cs};
+                       &w.dA, &w.dB, &w.dC, &w.f2, &w.rs, &w.cs};
     for (double **p : vecs) TRY(dalloc(h, p, L * ni));
     TRY(dalloc(h, &w.jv, L * (size_t)std::max(h->nnz, 1)));
     TRY(dalloc(h, &w.geo, L * 5 * ni));
@@ -341,12 +362,10 @@ extern "C" int vk_create(const vk_network *net, int max_cols, int max_layers, in
     TRY(dalloc(h, &w.status, max_cols));
     TRY(vk::init_kernels(h->net()) == cudaSuccess ? VK_OK
                                                   : fail(h, VK_ECUDA, "cudaFuncSetAttribute failed"));
-    TRY(vk::init_mixed_kernels(h->ni) == cudaSuccess ? VK_OK
+    TRY(vk::init_mixed_kernels(h->net()) == cudaSuccess ? VK_OK
                                                      : fail(h, VK_ECUDA, "cudaFuncSetAttribute (mixed) failed"));
-    TRY(vk::init_lureg_kernels(h->net()) == cudaSuccess ? VK_OK
-                                                     : fail(h, VK_ECUDA, "cudaFuncSetAttribute (LU) failed"));
-    TRY(vk::init_lu_tc(h->ni) == cudaSuccess ? VK_OK
-                                             : fail(h, VK_ECUDA, "cudaFuncSetAttribute (tensor-core LU) failed"));
+    TRY(vk::init_prep32(h->net()) == cudaSuccess && vk::init_lu32(h->ni) == cudaSuccess
+            ? VK_OK : fail(h, VK_ECUDA, "cudaFuncSetAttribute (FP32 LU) failed"));
     h->occ_rates = vk::rates_blocks_per_sm(h->net());
     h->occ_prep = vk::prep_blocks_per_sm(h->net());
     cudaGetLastError();                 // an occupancy query that failed leaves one CTA per layer
@@ -648,7 +667,8 @@ static void enqueue_attempt_kernels(vk_handle *h, const DevNet &net, const DevBa
         cudaEventRecord(h->ev_join, s2);
         DevBatch b32 = b;
         b32.active = w.act32;
-        vk::launch_lu_reg32(net, b32, w, s);
+        vk::launch_prep32(net, b32, w, s);
+        vk::launch_lu32(net, b32, w, s);
         if (timed) cudaEventRecord(h->ev[2], s);
         vk::launch_refine(net, b32, w, w.f, w.k1, w.y, w.yk2, h->max_refine, h->refine_tol, s);
         vk::launch_rates(net, b32, w.yk2, w.f2, nullptr, nullptr, nullptr, nullptr, w.k1, w.dt, w.geo, flags, false, s);
@@ -888,7 +908,7 @@ extern "C" int vk_set_launch(vk_handle *h, int kernel, int ctas_per_sm, int vari
     if (ctas_per_sm < 0 || ctas_per_sm > 8) return fail(h, VK_EINVAL, "ctas_per_sm must be 0..8");
     if (kernel == VK_TUNE_LU32 && variant != -1 &&
         (vk::lu32_tiling_cap(variant) == 0 || vk::lu32_tiling_cap(variant) < h->ni))
-        return fail(h, VK_EINVAL, "k_lu32 tiling " + std::to_string(variant) + " does not cover " +
+        return fail(h, VK_EINVAL, "LU32 variant " + std::to_string(variant) + " does not cover " +
                                       std::to_string(h->ni) + " species");
     if (h->stream) VK_CUDA(h, cudaStreamSynchronize(h->stream));
     drop_graph(h);                         // the captured loop has the old grids

@@ -85,6 +85,11 @@ struct DevNet {
     const double *jterm_nu;
     const int *jpos;
     const int *jrow, *jcol, *jrowptr, *jmap;
+    // Jacobian rows cut into pieces of similar length (k_refine): piece i sums
+    // entries [x, x + y); row s's pieces are rpc[rpcptr[s] .. rpcptr[s+1])
+    int npc;
+    const int2 *pc;
+    const int *rpcptr, *rpc;
     const double *compo;
     // the gather form (vk_network): pair order, source slots and coefficients,
     // extra products, derivative half terms, Jacobian gather terms
@@ -120,7 +125,7 @@ struct DevBatch {
     int cps;                   // resident CTAs per SM of the per-column kernels
                                // (0: each kernel's own default)
     int cps_k[VK_TUNE_N];      // per-kernel setting of vk_set_launch (0: cps)
-    int lu32_tiling;           // k_lu32 register tiling (-1: by ni)
+    int lu32_tiling;           // k_lu32 variant (-1: by ni)
     int grid_rates, grid_prep; // CTAs of the per-layer kernels k_rates / k_prep32:
                                // all of them resident at once, each striding over
                                // the layers (0: one CTA per layer)
@@ -214,7 +219,6 @@ struct Work {                  // per-handle device work buffers
     double *G;                 // [L][block_stride64(ni)] FP64 block inverses
     float *G32;                // [L][ni*ni] FP32 inverses of the scaled blocks (mixed mode)
     double *rs, *cs;           // [L][ni] power-of-two row / column scales (mixed mode)
-    double *r;                 // refinement residual
     double *f2;                // [L][ni] second-stage right-hand side (mixed mode)
     float *zf;                 // [L][ni] FP32 forward-sweep vector (mixed mode)
     float *wcf, *wcb;          // [L][ni] scaled couplings of the refinement sweeps (mixed mode)
@@ -232,7 +236,6 @@ struct Work {                  // per-handle device work buffers
     double *dt;                // [ncols]
     double *delta;             // [ncols]
     int *status;               // [ncols]  VK_* per column (singular pivot ...)
-    const void *tmap_d32;      // host: CUtensorMap over D32 as k_lu_tc's padded tiles
 };
 
 void launch_rates(const DevNet &net, const DevBatch &b, const double *y, double *f,
@@ -259,23 +262,15 @@ void launch_photo(const DevNet &net, const DevBatch &b, const PhotoDev &ph, cons
 void launch_photo_clear(const DevBatch &b, unsigned long long *change, cudaStream_t s);
 void launch_route(const DevBatch &b, const Work &w, cudaStream_t s);
 void launch_reset_route(const Work &w, int ncols, double route_dt0, cudaStream_t s);
-cudaError_t init_mixed_kernels(int n);
-cudaError_t init_lureg_kernels(const DevNet &net);
+cudaError_t init_mixed_kernels(const DevNet &net);
+cudaError_t init_prep32(const DevNet &net);
+cudaError_t init_lu32(int n);
 // Resident CTAs per SM of the per-layer kernels for a network (0: unknown);
 // call after the init_* functions have raised their shared-memory limits.
 int rates_blocks_per_sm(const DevNet &net);
 int prep_blocks_per_sm(const DevNet &net);
-void launch_lu_reg32(const DevNet &net, const DevBatch &b, const Work &w, cudaStream_t s);
-int lu32_tiling_cap(int tiling);     // largest block a k_lu32 tiling covers (0: none)
-// tensor-core factorisation (vk_lutc.cu): the LU32 tiling values that select
-// it with the one-warp panel and with the four-warp cooperative panel
-constexpr int VK_LU_TC = 4;
-constexpr int VK_LU_TC_COOP = 5;
-bool lu_tc_supported(int n);
-cudaError_t lu_tc_make_map(CUtensorMap *map, const float *D32, int n, int max_layers);
-void launch_lu_tc(const DevNet &net, const DevBatch &b, const Work &w, const CUtensorMap &map,
-                  bool coop, cudaStream_t s);
-size_t lu_tc_block_floats(int n);    // floats per layer of its padded scaled blocks
-cudaError_t init_lu_tc(int n);
+void launch_prep32(const DevNet &net, const DevBatch &b, const Work &w, cudaStream_t s);
+void launch_lu32(const DevNet &net, const DevBatch &b, const Work &w, cudaStream_t s);
+int lu32_tiling_cap(int tiling);     // largest block an LU32 variant covers (0: none)
 
 }  // namespace vk

@@ -29,60 +29,13 @@
 
 #include "vk_internal.cuh"
 #include "vk_gj.cuh"
+#include "vk_halves.cuh"
 #include "vk_lu64.cuh"
 #include "vk_tma.cuh"
 
 namespace vk {
 
 namespace {
-
-// The next unit of the queue: half-columns, the longest columns first.  In a
-// cluster every CTA gets rank 0's.
-template <bool CL>
-__device__ __forceinline__ int next_half(const DevBatch &b, int *s_unit, int rank, int csize) {
-    if (CL) {
-        cluster_sync_all();
-        if (rank == 0 && threadIdx.x == 0) {
-            const int u = (int)atomicAdd(b.queue, 1u);
-            const uint32_t la = smem_u32(s_unit);
-            for (int d = 0; d < csize; ++d)
-                asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(cluster_addr(la, (uint32_t)d)), "r"(u) : "memory");
-        }
-        cluster_sync_all();
-    } else {
-        __syncthreads();
-        if (threadIdx.x == 0) *s_unit = (int)atomicAdd(b.queue, 1u);
-        __syncthreads();
-    }
-    const int u = *s_unit;
-    return u < 2 * b.ncols ? u : -1;
-}
-
-// True for the second of a column's halves to get here; what the first wrote
-// before is then visible.  All threads call it (in a cluster: of every CTA).
-template <bool CL>
-__device__ __forceinline__ bool second_half(const DevBatch &b, int c, int *s_unit, int rank, int csize) {
-    __threadfence();
-    if (CL) {
-        cluster_sync_all();
-        if (rank == 0 && threadIdx.x == 0) {
-            const int a = (int)atomicAdd(b.queue + 1 + c, 1u);
-            __threadfence();
-            const uint32_t la = smem_u32(s_unit);
-            for (int d = 0; d < csize; ++d)
-                asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(cluster_addr(la, (uint32_t)d)), "r"(a) : "memory");
-        }
-        cluster_sync_all();
-    } else {
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            *s_unit = (int)atomicAdd(b.queue + 1 + c, 1u);
-            __threadfence();
-        }
-        __syncthreads();
-    }
-    return *s_unit == 1;
-}
 
 __host__ __device__ inline size_t lu64_smem(int n, int csize) {
     const int w = lu64_slice_max(n, csize);
@@ -228,19 +181,24 @@ k_lu64(DevNet net, DevBatch b, const double *__restrict__ jv, const double *__re
     if (CL) cluster_sync_all();            // no message is still on its way to a CTA that has left
 }
 
-// Shared memory of the FP64 sweeps: two mbarriers, nbuf blocks of the padded
-// stride, two vectors and the product's partial sums.  Two buffers (the next
-// block's copy overlaps this block's product) when they fit in a CTA's 227 KB,
-// else one (ni >~ 115).
+// Shared memory of the FP64 sweeps: the mbarriers, nbuf blocks of the padded
+// stride, two vectors and the product's partial sums.
+constexpr int kSweepBars = 12;
 static __host__ __device__ inline size_t sweep64_smem(int n, int nth, int nbuf) {
-    return 16 + (size_t)(nbuf * block_stride64(n) + 2 * n + (nth > n ? nth : n)) * sizeof(double);
+    return kSweepBars * 8 + (size_t)(nbuf * block_stride64(n) + 2 * n + (nth > n ? nth : n)) * sizeof(double);
 }
-static inline int sweep64_nbuf(int n) { return sweep64_smem(n, 256, 2) <= 232448 ? 2 : 1; }
+// Blocks in flight: as many as the CTA's share of the SM holds (a bulk copy of a
+// block takes longer than the product that uses it); one above ~115 species.
+static inline int sweep64_nbuf(int n, int ctas) {
+    int nb = kSweepBars;
+    while (nb > 1 && ctas * (sweep64_smem(n, 256, nb) + 1024) > 233472) --nb;
+    return nb;
+}
 
 // Copy k of a CTA's block stream lands in buffer k % nbuf and completes
 // phase (k / nbuf) & 1 of that buffer's mbarrier.
-__device__ __forceinline__ bool wait_copy(uint64_t *bar, unsigned k, int nbuf) {
-    return nbuf == 2 ? mbar_wait(&bar[k & 1], (k >> 1) & 1) : mbar_wait(&bar[0], k & 1);
+__device__ __forceinline__ bool wait_copy(uint64_t *bar, unsigned k, unsigned nbuf) {
+    return mbar_wait(&bar[k % nbuf], (k / nbuf) & 1u);
 }
 
 // After a bulk copy that never landed: wait (bounded) for the copies still in
@@ -255,9 +213,8 @@ __device__ __forceinline__ void drain_copies(uint64_t *bar, unsigned cnt, int v,
 //   z_m = G_m (rhs_m + dC_m o z_{m-1} + dB_m o z_{m+1});
 // else from the middle outwards, starting at out_m = z_m,
 //   out_j = z_j + G_j (coupling o out_prev), optional yk2 = y + out / r.
-// The inverses stream into shared memory by bulk copies in visit order,
-// double-buffered (nbuf = 2): the next block's copy runs during this block's
-// product.
+// The inverses stream into shared memory by bulk copies in visit order, nbuf
+// in flight.
 template <bool FWD>
 __global__ void __launch_bounds__(256)
 k_sweep64(DevNet net, DevBatch b, const double *G, const double *__restrict__ dB,
@@ -266,16 +223,15 @@ k_sweep64(DevNet net, DevBatch b, const double *G, const double *__restrict__ dB
     extern __shared__ __align__(16) unsigned char smb[];
     const int n = net.ni, gst = block_stride64(n);
     const int tid = threadIdx.x, nth = blockDim.x;
-    uint64_t *bar = reinterpret_cast<uint64_t *>(smb);      // [2]
-    double *Gbuf = reinterpret_cast<double *>(smb + 16);    // [nbuf][gst]
+    uint64_t *bar = reinterpret_cast<uint64_t *>(smb);      // [nbuf]
+    double *Gbuf = reinterpret_cast<double *>(smb + kSweepBars * 8);    // [nbuf][gst]
     double *xs = Gbuf + nbuf * gst;                         // [n] input of the visit
     double *xn = xs + n;                                    // [n] its result
     double *part = xn + n;                                  // [max(nth, n)]
     __shared__ int s_unit;
     const uint32_t bytes = (uint32_t)gst * sizeof(double);
     if (tid == 0) {
-        mbar_init(&bar[0], 1);
-        mbar_init(&bar[1], 1);
+        for (int i = 0; i < nbuf; ++i) mbar_init(&bar[i], 1);
         mbar_fence_init();
     }
     unsigned cnt = 0;              // copies this CTA consumed before the current unit
@@ -381,22 +337,10 @@ cudaError_t init_lu64(int n) {
         if (n >= kLu64MinCluster && lu64_smem(n, cs) <= 232448 && lu64_smem(n, cs) > scl) scl = lu64_smem(n, cs);
     cudaError_t e = raise_smem_limit(k_lu64<false>, lu64_smem(n, 1));
     if (e == cudaSuccess && scl) e = raise_smem_limit(k_lu64<true>, scl);
-    const size_t ssw = sweep64_smem(n, 256, sweep64_nbuf(n));
+    const size_t ssw = sweep64_smem(n, 256, sweep64_nbuf(n, 1));
     if (e == cudaSuccess) e = raise_smem_limit(k_sweep64<true>, ssw);
     if (e == cudaSuccess) e = raise_smem_limit(k_sweep64<false>, ssw);
     return e;
-}
-
-// Grid of a half-column kernel (column_grid's rule over 2 ncols units).
-static int half_grid(const DevBatch &b, int kernel, int cps_default) {
-    const int cps = b.cps_k[kernel] > 0 ? b.cps_k[kernel] : b.cps > 0 ? b.cps : cps_default;
-    const long long g = (long long)cps * b.nsm;
-    return (g > 0 && g < 2ll * b.ncols) ? (int)g : 2 * b.ncols;
-}
-
-// the queue position and the columns' arrival counts
-static void reset_queue(const DevBatch &b, cudaStream_t s) {
-    cudaMemsetAsync(b.queue, 0, (size_t)(1 + b.ncols) * sizeof(unsigned), s);
 }
 
 void launch_lu64(const DevNet &net, const DevBatch &b, const Work &w, cudaStream_t s) {
@@ -425,10 +369,13 @@ void launch_lu64(const DevNet &net, const DevBatch &b, const Work &w, cudaStream
                        cs);
 }
 
+// CTAs of a sweep an SM should hold
+static int sweep64_ctas(const DevBatch &b) { return 2 * b.ncols <= b.nsm ? 1 : 2; }
+
 void launch_fwd64(const DevNet &net, const DevBatch &b, const double *G, const double *dB,
                   const double *dC, const double *rhs, double *z, int *status, cudaStream_t s) {
     reset_queue(b, s);
-    const int nbuf = sweep64_nbuf(net.ni);
+    const int nbuf = sweep64_nbuf(net.ni, sweep64_ctas(b));
     k_sweep64<true><<<half_grid(b, VK_TUNE_SWEEP64, 2), 256, sweep64_smem(net.ni, 256, nbuf), s>>>(
         net, b, G, dB, dC, rhs, z, nullptr, nullptr, nullptr, status, nbuf);
 }
@@ -437,7 +384,7 @@ void launch_back64(const DevNet &net, const DevBatch &b, const double *G, const 
                    const double *dC, double *z, double *x, const double *y, double *yk2, int *status,
                    cudaStream_t s) {
     reset_queue(b, s);
-    const int nbuf = sweep64_nbuf(net.ni);
+    const int nbuf = sweep64_nbuf(net.ni, sweep64_ctas(b));
     k_sweep64<false><<<half_grid(b, VK_TUNE_SWEEP64, 2), 256, sweep64_smem(net.ni, 256, nbuf), s>>>(
         net, b, G, dB, dC, nullptr, z, x, y, yk2, status, nbuf);
 }

@@ -34,6 +34,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "vk_halves.cuh"
 #include "vk_tma.cuh"
 
 namespace vk {
@@ -49,19 +50,11 @@ __host__ __device__ inline int lu64_msg(int n) { return (n + 3) & ~1; }
 __host__ __device__ inline int lu64_slice(int n, int csize, int c) { return c * n / csize; }
 __host__ __device__ inline int lu64_slice_max(int n, int csize) { return (n + csize - 1) / csize; }
 
-__device__ __forceinline__ uint32_t cluster_addr(uint32_t a, uint32_t rank) {
-    uint32_t r;
-    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
-    return r;
-}
 // Copy of `bytes` from this CTA's shared memory into another CTA's of the
 // cluster, counted there on its mbarrier (all addresses 16-byte aligned).
 __device__ __forceinline__ void bulk_send(uint32_t dst, uint32_t src, uint32_t bytes, uint32_t bar) {
     asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                  ::"r"(dst), "r"(src), "r"(bytes), "r"(bar) : "memory");
-}
-__device__ __forceinline__ void cluster_sync_all() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 __device__ __forceinline__ uint32_t cluster_rank() {
     uint32_t r;
@@ -150,7 +143,7 @@ __device__ __forceinline__ void lu64_invert(const Lu64Mem &m, unsigned phase) {
             if (key == mx && recip64_edge_case(v)) x = recip64_edge(v);
             if (key == mx && key) m.xval[warp] = x;
         }
-        asm volatile("bar.sync 1, %0;" ::"r"(npt) : "memory");
+        asm volatile("barrier.sync 1, %0;" ::"r"(npt) : "memory");
         const uint4 ka = *reinterpret_cast<const uint4 *>(m.xkey), kb = *reinterpret_cast<const uint4 *>(m.xkey + 4);
         const unsigned best = max(max(max(ka.x, ka.y), max(ka.z, ka.w)), max(max(kb.x, kb.y), max(kb.z, kb.w)));
         int p = (best & 0x80000000u) ? 255 - (int)(best & 255u) : 256 - (int)best;
@@ -167,7 +160,7 @@ __device__ __forceinline__ void lu64_invert(const Lu64Mem &m, unsigned phase) {
                 if (recip64_edge_case(pv)) pinv = recip64_edge(pv);
                 if (lane == 0) m.xval[0] = pinv;
             }
-            asm volatile("bar.sync 1, %0;" ::"r"(npt) : "memory");
+            asm volatile("barrier.sync 1, %0;" ::"r"(npt) : "memory");
             pinv = m.xval[0];
         }
         if (r == p && (__double_as_longlong(v) & 0x7fffffffffffffffll) == 0) flag = 1;

@@ -159,6 +159,7 @@ k_gemm_bf16(int M, int N, int K, const __nv_bfloat16 *__restrict__ A, int chunkA
         asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
         __syncthreads();                                    // tile t landed; tile t - 1 is free
         fetch(t + STAGES - 1);
+        __syncwarp();                                       // ldmatrix and mma need the whole warp
         const __nv_bfloat16 *as = As + ((t - t0) % STAGES) * L::A, *bs = Bs + ((t - t0) % STAGES) * L::B;
 #pragma unroll
         for (int kk = 0; kk < BK; kk += 16) {
