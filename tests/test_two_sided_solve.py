@@ -70,7 +70,7 @@ def test_short_columns_and_block_sizes(name, nz):
         assert abs(delta[0] / r.delta - 1) <= 1e-6
 
 
-@pytest.mark.parametrize('name', ['CHO_thermo', 'NCHO_thermo'])
+@pytest.mark.parametrize('name', ['CHO_thermo', 'NCHO_thermo', 'TiSNCHO_photo', 'SYN150_photo'])
 def test_batch_size_does_not_change_a_column(name):
     net = Network.from_npz(os.path.join(GOLDEN, 'net_%s.npz' % name))
     items = [_item(net, name, nz, seed=nz) for nz in (9, 14, 21)]

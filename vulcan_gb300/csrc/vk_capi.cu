@@ -73,6 +73,7 @@ struct vk_handle {
     cudaStream_t stream2 = nullptr;     // FP64 branch of a mixed attempt (routed columns)
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     int nsm = 0;                        // SMs of the device
+    int ncl_lu[3] = {}, ncl_sweep[3] = {};      // clusters it holds at once
     int cps = 0;                        // VK_CTAS_PER_SM override (0: kernel defaults)
     int cps_k[VK_TUNE_N] = {0, 0, 0, 0}; // vk_set_launch: CTAs per SM per kernel
     int lu32_tiling = -1;               // vk_set_launch: k_lu32 variant (-1: by ni)
@@ -115,6 +116,10 @@ struct vk_handle {
         b.order = d_order;
         b.queue = d_queue;
         b.nsm = nsm;
+        for (int i = 0; i < 3; ++i) {
+            b.ncl_lu[i] = ncl_lu[i];
+            b.ncl_sweep[i] = ncl_sweep[i];
+        }
         b.cps = cps;
         for (int i = 0; i < VK_TUNE_N; ++i) b.cps_k[i] = cps_k[i];
         b.lu32_tiling = lu32_tiling;
@@ -366,6 +371,7 @@ extern "C" int vk_create(const vk_network *net, int max_cols, int max_layers, in
                                                      : fail(h, VK_ECUDA, "cudaFuncSetAttribute (mixed) failed"));
     TRY(vk::init_prep32(h->net()) == cudaSuccess && vk::init_lu32(h->ni) == cudaSuccess
             ? VK_OK : fail(h, VK_ECUDA, "cudaFuncSetAttribute (FP32 LU) failed"));
+    vk::cluster_limits(h->ni, h->ncl_lu, h->ncl_sweep);
     h->occ_rates = vk::rates_blocks_per_sm(h->net());
     h->occ_prep = vk::prep_blocks_per_sm(h->net());
     cudaGetLastError();                 // an occupancy query that failed leaves one CTA per layer

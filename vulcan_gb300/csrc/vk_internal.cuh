@@ -122,6 +122,7 @@ struct DevBatch {
     unsigned *queue;           // [1 + ncols] next queue position, then per column how many of
                                //  its halves are done (zeroed before each launch)
     int nsm;                   // SMs of the device
+    int ncl_lu[3], ncl_sweep[3];    // clusters of 2, 4, 8 CTAs it holds at once (vk_lu64.cu)
     int cps;                   // resident CTAs per SM of the per-column kernels
                                // (0: each kernel's own default)
     int cps_k[VK_TUNE_N];      // per-kernel setting of vk_set_launch (0: cps)
@@ -243,7 +244,13 @@ void launch_rates(const DevNet &net, const DevBatch &b, const double *y, double 
                   const double *dt, const double *geo, int flags, bool with_jac, cudaStream_t s);
 void launch_geometry(const DevNet &net, const DevBatch &b, double *geo, int flags, cudaStream_t s);
 cudaError_t init_lu64(int n);
+void cluster_limits(int n, int lu[3], int sweep[3]);
 void launch_lu64(const DevNet &net, const DevBatch &b, const Work &w, cudaStream_t s);
+// One column of given blocks (sizes and words: vk_lu64.cu).
+constexpr int kSolve64Words = 8;
+cudaError_t init_solve64(int nmax);
+cudaError_t launch_solve64(int nz, int n, const double *D, const double *lo, const double *up, const double *rhs,
+                           double *x, double *G, double *z, int *words, int mid, cudaStream_t s);
 void launch_fwd64(const DevNet &net, const DevBatch &b, const double *G, const double *dB,
                   const double *dC, const double *rhs, double *z, int *status, cudaStream_t s);
 void launch_back64(const DevNet &net, const DevBatch &b, const double *G, const double *dB,

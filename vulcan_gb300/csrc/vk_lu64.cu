@@ -10,17 +10,17 @@
 //               D'_j = D_j - diag(dB_j) G_{j+1} diag(dC_{j+1});
 //             whoever finishes a column's second half inverts its middle
 //             layer, which has both terms.  D_j = c0 I - J_j - diag(dA_j).
-//   k_fwd64   z_j = G_j (b_j + coupling o z_prev) along both halves; the second
+//   k_sweep64<true>   z_j = G_j (b_j + coupling o z_prev) along both halves; the second
 //             half to finish does the middle: x_m = z_m.
-//   k_back64  x_j = z_j + G_j (coupling o x_next) from the middle outwards.
+//   k_sweep64<false>  x_j = z_j + G_j (coupling o x_next) from the middle outwards.
 //
 // k_lu64 is bound by the FP64 unit when the columns fill the chip (one
 // warp-wide FP64 instruction per 19 cycles and SM, measured) and by the chain
 // of dependent pivots (vk_lu64.cuh) when they do not: then the CTAs of a
 // cluster share each block.  Measured against the one-sided factorisation,
 // one CTA per column, that it replaced (ms, GB300): one CHO column of 100
-// layers 6.1 -> 1.6, one NCHO column of 150 layers 21.4 -> 4.4, 64 uneven NCHO
-// columns 28.0 -> 12.5, 512 50.6 -> 49.4.  The sweeps are bound by the FP64
+// layers 6.1 -> 1.5, one NCHO column of 150 layers 21.4 -> 4.2, 64 uneven NCHO
+// columns 28.0 -> 12.2, 512 50.6 -> 46.0.  The sweeps are bound by the FP64
 // products of a layer and the latency between dependent layers.
 //
 // Reference: the banded LU of the Ros2 LHS, op.py:2913-2929.
@@ -28,7 +28,6 @@
 #include <math.h>
 
 #include "vk_internal.cuh"
-#include "vk_gj.cuh"
 #include "vk_halves.cuh"
 #include "vk_lu64.cuh"
 #include "vk_tma.cuh"
@@ -36,6 +35,8 @@
 namespace vk {
 
 namespace {
+
+constexpr size_t kMaxSmem = 232448;    // dynamic shared memory of a CTA
 
 __host__ __device__ inline size_t lu64_smem(int n, int csize) {
     const int w = lu64_slice_max(n, csize);
@@ -45,14 +46,17 @@ __host__ __device__ inline size_t lu64_smem(int n, int csize) {
 
 }  // namespace
 
-template <bool CL>
-__global__ void __launch_bounds__(352, CL ? 1 : 2)
+// DENSE: the blocks are given, jv = D [layer][n][n], and so are the couplings
+// (their sign cancels in the Schur terms); the inverses are packed (stride n n).
+// mid1: the middle layer, nz / 2 if negative.
+template <bool CL, bool DENSE>
+__global__ void __launch_bounds__(CL ? 384 : 544, CL ? 1 : 2)
 k_lu64(DevNet net, DevBatch b, const double *__restrict__ jv, const double *__restrict__ dA,
        const double *__restrict__ dB, const double *__restrict__ dC,
-       const double *__restrict__ dt, double *G, int *status, int csize) {
+       const double *__restrict__ dt, double *G, int *status, int csize, int mid1) {
     extern __shared__ __align__(16) double sm[];
     __shared__ int s_unit, s_sing, s_dead;
-    const int n = net.ni, gst = block_stride64(n);
+    const int n = net.ni, gst = DENSE ? n * n : block_stride64(n);
     const int tid = threadIdx.x, nth = blockDim.x;
     Lu64Mem m;
     m.n = n;
@@ -88,9 +92,9 @@ k_lu64(DevNet net, DevBatch b, const double *__restrict__ jv, const double *__re
     for (int u; (u = next_half<CL>(b, &s_unit, m.rank, m.csize)) >= 0;) {
         const int c = b.order[u >> 1], half = u & 1;
         if (b.active && !b.active[c]) continue;
-        const int l0 = b.col_off[c], nz = b.col_end[c] - l0, mid = nz / 2;
+        const int l0 = b.col_off[c], nz = b.col_end[c] - l0, mid = mid1 >= 0 ? mid1 : nz / 2;
         const int cnt = half ? nz - 1 - mid : mid;
-        const double cdt = 1.0 / (R_ROS * dt[c]);
+        const double cdt = DENSE ? 0.0 : 1.0 / (R_ROS * dt[c]);
         if (tid == 0) s_sing = 0;
         for (int t = tid; t < n; t += nth) { m.rowid[t] = t; m.colid[t] = t; }
         __syncthreads();
@@ -101,11 +105,12 @@ k_lu64(DevNet net, DevBatch b, const double *__restrict__ jv, const double *__re
             const int j = middle ? mid : (half ? nz - 1 - t : t);
             const size_t l = (size_t)l0 + j;
             const bool build = t < cnt || middle;
+            const double *Dl = DENSE ? jv + l * gst : nullptr;
             if (build) {
                 const double *rf = half ? dB + l * n : dC + l * n;
                 const double *cf = half ? dC + (l + 1) * n : dB + (l - 1) * n;
                 for (int q = tid; q < n; q += nth) {
-                    diag[q] = cdt - dA[l * n + q];
+                    if (!DENSE) diag[q] = cdt - dA[l * n + q];
                     if (t > 0 && !middle) {
                         rowf[q] = -rf[m.rowid[q]] * m.srow[q];
                         colf[q] = cf[m.colid[q]];
@@ -116,18 +121,19 @@ k_lu64(DevNet net, DevBatch b, const double *__restrict__ jv, const double *__re
             if (middle) {
                 // natural order; both neighbours' inverses from global memory
                 const double *Gd = G + (l - 1) * gst, *Gu = G + (l + 1) * gst;
-                const bool up = mid + 1 < nz;
+                const bool down = mid > 0, up = mid + 1 < nz;
                 for (int e = tid; e < ne; e += nth) {
                     const int r = e / w, q = c0s + e - r * w;
-                    double v = -dC[l * n + r] * __ldcg(Gd + r * n + q) * dB[(l - 1) * n + q];
+                    double v = down ? -dC[l * n + r] * __ldcg(Gd + r * n + q) * dB[(l - 1) * n + q] : 0.0;
                     if (up) v -= dB[l * n + r] * __ldcg(Gu + r * n + q) * dC[(l + 1) * n + q];
-                    if (r == q) v += diag[r];
+                    if (DENSE) v += Dl[r * n + q];
+                    else if (r == q) v += diag[r];
                     m.S[e] = v;
                 }
             } else if (t == 0) {
                 if (build) for (int e = tid; e < ne; e += nth) {
                     const int r = e / w, q = c0s + e - r * w;
-                    m.S[e] = r == q ? diag[r] : 0.0;
+                    m.S[e] = DENSE ? Dl[r * n + q] : r == q ? diag[r] : 0.0;
                 }
             } else {
                 // store the previous layer's inverse and replace it by this layer's Schur term
@@ -139,21 +145,24 @@ k_lu64(DevNet net, DevBatch b, const double *__restrict__ jv, const double *__re
                     Gp[ri * n + ci] = s * m.srow[r];
                     if (build) {
                         double v = s * rowf[r] * colf[q];
-                        if (ri == ci) v += diag[ri];
+                        if (DENSE) v += Dl[ri * n + ci];
+                        else if (ri == ci) v += diag[ri];
                         m.S[e] = v;
                     }
                 }
             }
             if (build) {
-                for (int q = tid; q < n; q += nth) {
-                    rowpos[m.rowid[q]] = q;
-                    colpos[m.colid[q]] = q - c0s;
-                }
-                __syncthreads();
-                const double *jl = jv + l * net.nnz;
-                for (int e = tid; e < net.nnz; e += nth) {
-                    const int q = colpos[net.jcol[e]];
-                    if (!CL || (unsigned)q < (unsigned)w) m.S[rowpos[net.jrow[e]] * w + q] += jl[e];
+                if (!DENSE) {
+                    for (int q = tid; q < n; q += nth) {
+                        rowpos[m.rowid[q]] = q;
+                        colpos[m.colid[q]] = q - c0s;
+                    }
+                    __syncthreads();
+                    const double *jl = jv + l * net.nnz;
+                    for (int e = tid; e < net.nnz; e += nth) {
+                        const int q = colpos[net.jcol[e]];
+                        if (!CL || (unsigned)q < (unsigned)w) m.S[rowpos[net.jrow[e]] * w + q] += jl[e];
+                    }
                 }
                 __syncthreads();
                 lu64_invert<CL>(m, phase);
@@ -181,17 +190,39 @@ k_lu64(DevNet net, DevBatch b, const double *__restrict__ jv, const double *__re
     if (CL) cluster_sync_all();            // no message is still on its way to a CTA that has left
 }
 
-// Shared memory of the FP64 sweeps: the mbarriers, nbuf blocks of the padded
-// stride, two vectors and the product's partial sums.
-constexpr int kSweepBars = 12;
-static __host__ __device__ inline size_t sweep64_smem(int n, int nth, int nbuf) {
-    return kSweepBars * 8 + (size_t)(nbuf * block_stride64(n) + 2 * n + (nth > n ? nth : n)) * sizeof(double);
+// One FP64 sweep over half-columns.  FWD: towards the middle,
+//   z_j = G_j (rhs_j + coupling o z_prev), the second half to finish adding
+//   z_m = G_m (rhs_m + dC_m o z_{m-1} + dB_m o z_{m+1});
+// else from the middle outwards, starting at out_m = z_m,
+//   out_j = z_j + G_j (coupling o out_prev), optional yk2 = y + out / r.
+// A row's product is the same sums in the same order in both kernels below:
+// eight parts, part p over the columns p, p + 8, .., combined
+// ((p0 + p4) + (p1 + p5)) + ((p2 + p6) + (p3 + p7)).
+// The lane that ends up with row r of a result also computes row r of the next
+// visit's input, so a visit has one barrier; y + out / r (a division each) is
+// formed in a parallel pass after the half.
+
+// y + out / r of the layers [j0, j1) of a half
+__device__ __forceinline__ void yk2_pass(size_t e0, int ne, int first, int step, const double *__restrict__ y,
+                                         const double *out, double *__restrict__ yk2) {
+#pragma unroll 2
+    for (int e = first; e < ne; e += step) yk2[e0 + e] = y[e0 + e] + out[e0 + e] / R_ROS;
 }
-// Blocks in flight: as many as the CTA's share of the SM holds (a bulk copy of a
-// block takes longer than the product that uses it); one above ~115 species.
-static inline int sweep64_nbuf(int n, int ctas) {
-    int nb = kSweepBars;
-    while (nb > 1 && ctas * (sweep64_smem(n, 256, nb) + 1024) > 233472) --nb;
+
+// --- one CTA per half-column, four lanes a row (two parts each).  The
+// inverses come by bulk copies in visit order, nbuf in flight, the row vectors
+// by cp.async two visits ahead.  Bound by the FP64 unit with many columns
+// (two solves of 512 NCHO columns 5.4 -> 5.1 ms against three barriers a visit
+// and a division by r in it, 64 columns 1.49 -> 1.12) and by the chain of visits with few.
+constexpr int kSweepBars = 8;
+__host__ __device__ inline int sweep64_threads(int n) { return (4 * n + 31) / 32 * 32; }
+__host__ __device__ inline size_t sweep64_smem(int n, int nbuf) {
+    return kSweepBars * 8 + (size_t)(nbuf * block_stride64(n) + 8 * n) * sizeof(double);
+}
+// Blocks in flight: as many as the CTA's share of the SM holds; one above ~115 species.
+inline int sweep64_nbuf(int n, int ctas) {
+    int nb = 4;
+    while (nb > 1 && ctas * (sweep64_smem(n, nb) + 1100) > 233472) --nb;
     return nb;
 }
 
@@ -208,15 +239,8 @@ __device__ __forceinline__ void drain_copies(uint64_t *bar, unsigned cnt, int v,
     for (int u = v; u < last; ++u) wait_copy(bar, cnt + (unsigned)u, nbuf);
 }
 
-// One sweep over half-columns.  FWD: towards the middle,
-//   z_j = G_j (rhs_j + coupling o z_prev), the second half to finish adding
-//   z_m = G_m (rhs_m + dC_m o z_{m-1} + dB_m o z_{m+1});
-// else from the middle outwards, starting at out_m = z_m,
-//   out_j = z_j + G_j (coupling o out_prev), optional yk2 = y + out / r.
-// The inverses stream into shared memory by bulk copies in visit order, nbuf
-// in flight.
 template <bool FWD>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(640)
 k_sweep64(DevNet net, DevBatch b, const double *G, const double *__restrict__ dB,
           const double *__restrict__ dC, const double *__restrict__ rhs, double *z, double *out,
           const double *__restrict__ y, double *__restrict__ yk2, int *__restrict__ status, int nbuf) {
@@ -225,11 +249,12 @@ k_sweep64(DevNet net, DevBatch b, const double *G, const double *__restrict__ dB
     const int tid = threadIdx.x, nth = blockDim.x;
     uint64_t *bar = reinterpret_cast<uint64_t *>(smb);      // [nbuf]
     double *Gbuf = reinterpret_cast<double *>(smb + kSweepBars * 8);    // [nbuf][gst]
-    double *xs = Gbuf + nbuf * gst;                         // [n] input of the visit
-    double *xn = xs + n;                                    // [n] its result
-    double *part = xn + n;                                  // [max(nth, n)]
+    double *xs = Gbuf + nbuf * gst;                         // [2][n] inputs of two visits
+    double *vec = xs + 2 * n;                               // [3][2][n] (coupling, rhs or z) of three visits
     __shared__ int s_unit;
     const uint32_t bytes = (uint32_t)gst * sizeof(double);
+    const int row = tid >> 2, part = tid & 3;
+    const bool rowt = row < n, lead = rowt && part == 0;
     if (tid == 0) {
         for (int i = 0; i < nbuf; ++i) mbar_init(&bar[i], 1);
         mbar_fence_init();
@@ -239,71 +264,103 @@ k_sweep64(DevNet net, DevBatch b, const double *G, const double *__restrict__ dB
         const int c = b.order[u >> 1], half = u & 1;
         if (b.active && !b.active[c]) continue;
         const int l0 = b.col_off[c], nz = b.col_end[c] - l0, mid = nz / 2;
-        int nvis = half ? nz - 1 - mid : mid;
-        auto layer_of = [&](int v) {
-            if (FWD) return half ? nz - 1 - v : v;
-            return half ? mid + 1 + v : mid - 1 - v;
-        };
-        auto issue = [&](int v, int j) {                    // thread 0
+        const int nvis = half ? nz - 1 - mid : mid;
+        const int first = FWD ? (half ? nz - 1 : 0) : (half ? mid + 1 : mid - 1);
+        const int step = FWD == (half != 0) ? -1 : 1;
+        const double *cpl = FWD == (half != 0) ? dB : dC;
+        const size_t e1 = ((size_t)l0 + first) * n;         // first layer visited
+        const ptrdiff_t es = (ptrdiff_t)step * n;
+        auto issue = [&](int v) {                           // thread 0
             const unsigned k = cnt + (unsigned)v, bi = k % (unsigned)nbuf;
-            tma_load_1d(Gbuf + bi * gst, G + ((size_t)l0 + j) * gst, bytes, &bar[bi]);
+            tma_load_1d(Gbuf + bi * gst, G + ((size_t)l0 + first + step * v) * gst, bytes, &bar[bi]);
+        };
+        // the lead's own vectors: of visit v's result (z) and of the input that follows it
+        auto fetch = [&](int v) {
+            if (lead && v < nvis) {
+                double *s = vec + (v % 3) * 2 * n + row;
+                const size_t e = e1 + es * v + row;
+                if (v + 1 < nvis) cp_async8(s, cpl + e + es);
+                if (!FWD) cp_async8(s + n, z + e);
+                else if (v + 1 < nvis) cp_async8(s + n, rhs + e + es);
+            }
+            cp_async_commit();
         };
         if (tid == 0)
-            for (int v = 0; v < nbuf && v < nvis; ++v) issue(v, layer_of(v));
-        if (!FWD) {
-            const size_t l = (size_t)l0 + mid;
-            for (int t = tid; t < n; t += nth) {
-                const double xv = z[l * n + t];
-                xn[t] = xv;
-                if (half == 0) {
-                    out[l * n + t] = xv;
-                    if (yk2) yk2[l * n + t] = y[l * n + t] + xv / R_ROS;
+            for (int v = 0; v < nbuf && v < nvis; ++v) issue(v);
+        fetch(0);
+        fetch(1);
+        int p = 0, v = 0, timed_out = 0;
+        if (FWD) {
+            if (lead && nvis > 0) xs[row] = rhs[e1 + row];
+        } else {
+            const size_t em = ((size_t)l0 + mid) * n;
+            if (lead) {
+                const double xv = z[em + row];
+                if (half == 0) out[em + row] = xv;
+                if (nvis > 0) xs[row] = cpl[e1 + row] * xv;
+            }
+        }
+        // rows of the product of block k with the current input
+        auto product = [&](unsigned k) {
+            const double *g = Gbuf + (k % (unsigned)nbuf) * gst + row * n, *xin = xs + p * n;
+            double a = 0.0, d = 0.0;
+            if (rowt) {
+                int q = part;
+                for (; q + 12 < n; q += 16) {
+                    const double g0 = g[q], g1 = g[q + 4], g2 = g[q + 8], g3 = g[q + 12];
+                    const double x0 = xin[q], x1 = xin[q + 4], x2 = xin[q + 8], x3 = xin[q + 12];
+                    a = __fma_rn(g0, x0, a);
+                    d = __fma_rn(g1, x1, d);
+                    a = __fma_rn(g2, x2, a);
+                    d = __fma_rn(g3, x3, d);
+                }
+                for (; q < n; q += 8) {
+                    a = __fma_rn(g[q], xin[q], a);
+                    if (q + 4 < n) d = __fma_rn(g[q + 4], xin[q + 4], d);
                 }
             }
-            __syncthreads();
-        }
-        int v = 0, timed_out = 0;
+            a += d;
+            __syncwarp();
+            a += __shfl_xor_sync(0xffffffffu, a, 1);
+            return a + __shfl_xor_sync(0xffffffffu, a, 2);
+        };
         for (; v < nvis; ++v) {
-            const int j = layer_of(v);
-            const size_t l = (size_t)l0 + j;
-            // the input: this thread's xn entry is the one it wrote itself (FWD:
-            // it reads the previous result, visible since the product's barrier)
-            for (int t = tid; t < n; t += nth) {
-                if (FWD) {
-                    const double cpl = v == 0 ? 0.0 : (half ? dB[l * n + t] : dC[l * n + t]) * xn[t];
-                    xs[t] = rhs[l * n + t] + cpl;
-                } else {
-                    xs[t] = (half ? dC[l * n + t] : dB[l * n + t]) * xn[t];
-                }
+            if (nbuf == 1 && v > 0) {                       // the one buffer, when all have read it
+                __syncthreads();
+                if (tid == 0) issue(v);
             }
-            const unsigned k = cnt + (unsigned)v;
-            const bool ok = wait_copy(bar, k, nbuf);
+            const bool ok = wait_copy(bar, cnt + (unsigned)v, nbuf);
             if (__syncthreads_or(!ok)) { timed_out = 1; break; }
-            matvec_f64(Gbuf + (k % (unsigned)nbuf) * gst, n, xs, part, xn, FWD ? nullptr : z + l * n);
-            if (tid == 0 && v + nbuf < nvis) issue(v + nbuf, layer_of(v + nbuf));   // the buffer just read is free
-            for (int t = tid; t < n; t += nth) {
-                const double xv = xn[t];
-                if (FWD) {
-                    z[l * n + t] = xv;
-                } else {
-                    out[l * n + t] = xv;
-                    if (yk2) yk2[l * n + t] = y[l * n + t] + xv / R_ROS;
-                }
+            if (tid == 0 && nbuf > 1 && v > 0 && v - 1 + nbuf < nvis) issue(v - 1 + nbuf);      // its buffer is free
+            cp_async_wait<1>();
+            double r = product(cnt + (unsigned)v);
+            if (lead) {
+                const double *s = vec + (v % 3) * 2 * n + row;
+                if (!FWD) r += s[n];
+                (FWD ? z : out)[e1 + es * v + row] = r;
+                if (v + 1 < nvis) xs[(p ^ 1) * n + row] = FWD ? __fma_rn(s[0], r, s[n]) : s[0] * r;
             }
+            p ^= 1;
+            fetch(v + 2);
         }
+        cp_async_wait<0>();
         if (timed_out) {
-            drain_copies(bar, cnt, v, nvis < v + nbuf ? nvis : v + nbuf, nbuf);
+            // issued so far: up to visit v - 2 + nbuf, v at least
+            const int last = v == 0 || nbuf == 1 ? v + nbuf : v - 1 + nbuf;
+            drain_copies(bar, cnt, v, nvis < last ? nvis : last, nbuf);
             if (tid == 0) status[c] = VK_ETIMEOUT;
             return;
         }
         cnt += (unsigned)nvis;
         if (FWD && second_half<false>(b, c, &s_unit, 0, 1)) {
-            const size_t l = (size_t)l0 + mid;
-            if (tid == 0) issue(0, mid);
-            for (int t = tid; t < n; t += nth) {
-                double s = rhs[l * n + t] + dC[l * n + t] * __ldcg(z + (l - 1) * n + t);
-                if (mid + 1 < nz) s += dB[l * n + t] * __ldcg(z + (l + 1) * n + t);
-                xs[t] = s;
+            const size_t e = ((size_t)l0 + mid) * n + row;
+            if (tid == 0) tma_load_1d(Gbuf + (cnt % (unsigned)nbuf) * gst, G + ((size_t)l0 + mid) * gst, bytes,
+                                      &bar[cnt % (unsigned)nbuf]);
+            if (lead) {
+                double s = rhs[e];
+                if (mid > 0) s = __fma_rn(dC[e], __ldcg(z + e - n), s);
+                if (mid + 1 < nz) s = __fma_rn(dB[e], __ldcg(z + e + n), s);
+                xs[p * n + row] = s;
             }
             const bool ok = wait_copy(bar, cnt, nbuf);
             if (__syncthreads_or(!ok)) {
@@ -311,82 +368,329 @@ k_sweep64(DevNet net, DevBatch b, const double *G, const double *__restrict__ dB
                 if (tid == 0) status[c] = VK_ETIMEOUT;
                 return;
             }
-            matvec_f64(Gbuf + (cnt % (unsigned)nbuf) * gst, n, xs, part, xn, nullptr);
-            for (int t = tid; t < n; t += nth) z[l * n + t] = xn[t];
+            const double r = product(cnt);
+            if (lead) z[e] = r;
             cnt += 1;
+        }
+        if (!FWD && yk2) {
+            __syncthreads();
+            const int j0 = half ? mid + 1 : 0, j1 = half ? nz : mid + 1;
+            yk2_pass(((size_t)l0 + j0) * n, (j1 - j0) * n, tid, nth, y, out, yk2);
         }
     }
 }
 
+// --- a cluster per half-column: CTA c has the rows [c n / cs, (c + 1) n / cs),
+// eight lanes each (one part), whose blocks a lane copies itself, kSweepAhead
+// visits ahead (its own copies need no barrier).  The eight lanes
+// send the row of the next input to one CTA each; one cluster barrier a visit.
+// Results are kept in shared memory for kSweepHist visits: a store to global
+// memory before the barrier would have to be acknowledged there.
+// Bound by the chain of a visit: n / 8 dependent FMAs, three exchanges and the
+// barrier. 
+// Two solves of one NCHO column of 150 layers 0.89 -> 0.53 ms (one CTA per half before).
+constexpr int kSweepAhead = 4;
+constexpr int kSweepHist = 32;          // visits whose results wait in shared memory
+__host__ __device__ inline int sweep64c_threads(int n, int cs) { return (8 * lu64_slice_max(n, cs) + 31) / 32 * 32; }
+__host__ __device__ inline size_t sweep64c_smem(int n, int cs) {
+    return (size_t)(kSweepAhead * ((n + 7) / 8 + 2) * sweep64c_threads(n, cs) + 2 * n +
+                    kSweepHist * lu64_slice_max(n, cs)) * sizeof(double);
+}
+
+// sgn: sign of the couplings (+1: the solver's, A = D - dC - dB; -1: A = D + lower +
+// upper); gst: stride of the blocks; mid1: the middle layer, nz / 2 if negative;
+// a column whose status is not 0 is left alone if skip.
+template <bool FWD>
+__global__ void __launch_bounds__(640)
+k_sweep64c(int n, int gst, DevBatch b, const double *G, const double *__restrict__ dB,
+           const double *__restrict__ dC, double sgn, const double *__restrict__ rhs, double *z, double *out,
+           const double *__restrict__ y, double *__restrict__ yk2, const int *__restrict__ status, int csize,
+           int mid1, int skip) {
+    extern __shared__ __align__(16) double smc[];
+    __shared__ int s_unit;
+    const int tid = threadIdx.x, nth = blockDim.x, K = (n + 7) / 8;
+    double *ring = smc;                                     // [ahead][K][nth] each lane's part of its row
+    double *vec = ring + kSweepAhead * K * nth;             // [ahead][2][nth] coupling, rhs or z
+    double *xs = vec + kSweepAhead * 2 * nth;               // [2][n] inputs of two visits
+    double *hist = xs + 2 * n;                              // [kSweepHist][rows] results
+    const int rank = (int)cluster_rank(), u = (int)blockIdx.x / csize;
+    const int r0 = lu64_slice(n, csize, rank), r1 = lu64_slice(n, csize, rank + 1);
+    const int row = r0 + (tid >> 3), part = tid & 7;
+    const bool rowt = row < r1, lead = rowt && part == 0;
+    const int c = b.order[u >> 1], half = u & 1;
+    // (the same for every CTA of the cluster)
+    if ((b.active && !b.active[c]) || (skip && status[c])) return;
+    const int l0 = b.col_off[c], nz = b.col_end[c] - l0, mid = mid1 >= 0 ? mid1 : nz / 2;
+    const int nvis = half ? nz - 1 - mid : mid;
+    const int first = FWD ? (half ? nz - 1 : 0) : (half ? mid + 1 : mid - 1);
+    const int step = FWD == (half != 0) ? -1 : 1;
+    const double *cpl = FWD == (half != 0) ? dB : dC;
+    const size_t e1 = ((size_t)l0 + first) * n;
+    const ptrdiff_t es = (ptrdiff_t)step * n;
+    const int nfetch = FWD ? nvis + 1 : nvis;               // FWD: the middle's block too
+    auto fetch = [&](int v) {
+        if (rowt && v < nfetch) {
+            const int s = v % kSweepAhead;
+            const double *g = G + ((size_t)l0 + first + step * v) * gst + (size_t)row * n + part;
+            for (int i = 0; part + 8 * i < n; ++i) cp_async8(ring + (s * K + i) * nth + tid, g + 8 * i);
+            if (v < nvis) {
+                const size_t e = e1 + es * v + row;
+                if (v + 1 < nvis) cp_async8(vec + (s * 2) * nth + tid, cpl + e + es);
+                if (!FWD) cp_async8(vec + (s * 2 + 1) * nth + tid, z + e);
+                else if (v + 1 < nvis) cp_async8(vec + (s * 2 + 1) * nth + tid, rhs + e + es);
+            }
+        }
+        cp_async_commit();
+    };
+    for (int v = 0; v < kSweepAhead - 1; ++v) fetch(v);
+    if (FWD) {
+        if (nvis > 0)
+            for (int t = tid; t < n; t += nth) xs[t] = rhs[e1 + t];
+    } else {
+        const size_t em = ((size_t)l0 + mid) * n;
+        if (nvis > 0)
+            for (int t = tid; t < n; t += nth) xs[t] = (sgn * cpl[e1 + t]) * z[em + t];
+        if (half == 0 && lead) out[em + row] = z[em + row];
+    }
+    __syncthreads();
+    int p = 0;
+    auto product = [&](int v) {
+        const double *g = ring + (v % kSweepAhead) * K * nth + tid, *xin = xs + p * n;
+        double a = 0.0;
+        if (rowt) {
+            int i = 0, q = part;
+            for (; q + 24 < n; q += 32, i += 4) {
+                const double g0 = g[i * nth], g1 = g[(i + 1) * nth], g2 = g[(i + 2) * nth], g3 = g[(i + 3) * nth];
+                const double x0 = xin[q], x1 = xin[q + 8], x2 = xin[q + 16], x3 = xin[q + 24];
+                a = __fma_rn(g0, x0, a);
+                a = __fma_rn(g1, x1, a);
+                a = __fma_rn(g2, x2, a);
+                a = __fma_rn(g3, x3, a);
+            }
+            for (; q < n; q += 8, ++i) a = __fma_rn(g[i * nth], xin[q], a);
+        }
+        __syncwarp();
+        a += __shfl_xor_sync(0xffffffffu, a, 4);
+        a += __shfl_xor_sync(0xffffffffu, a, 1);
+        return a + __shfl_xor_sync(0xffffffffu, a, 2);
+    };
+    const uint32_t peer = part < csize ? cluster_addr(smem_u32(xs), (uint32_t)part) : 0u;
+    cluster_sync_all();                                     // every CTA of the cluster runs
+    for (int v = 0; v < nvis; ++v) {
+        cp_async_wait<kSweepAhead - 2>();
+        double r = product(v);
+        if (rowt) {
+            const double *s = vec + (v % kSweepAhead) * 2 * nth + tid;
+            if (!FWD) r += s[nth];
+            if (v + 1 < nvis && part < csize) {
+                const double f = sgn * s[0], xn = FWD ? __fma_rn(f, r, s[nth]) : f * r;
+                asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(peer + (uint32_t)((p ^ 1) * n + row) * 8u), "d"(xn)
+                             : "memory");
+            }
+            if (part == 0) hist[(v % kSweepHist) * (r1 - r0) + row - r0] = r;
+        }
+        asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+        fetch(v + kSweepAhead - 1);
+        if (v + 1 == nvis || (v + 1) % kSweepHist == 0) {
+            __syncwarp();
+            const int v0 = v - v % kSweepHist;
+            if (rowt)
+                for (int t = v0 + part; t <= v; t += 8)
+                    (FWD ? z : out)[e1 + es * t + row] = hist[(t - v0) * (r1 - r0) + row - r0];
+            __syncwarp();
+        }
+        asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+        p ^= 1;
+    }
+    cp_async_wait<0>();
+    if (FWD) {
+        if (second_half<true>(b, c, &s_unit, rank, csize)) {
+            const size_t em = ((size_t)l0 + mid) * n;
+            for (int t = tid; t < n; t += nth) {
+                double s = rhs[em + t];
+                if (mid > 0) s = __fma_rn(sgn * dC[em + t], __ldcg(z + em - n + t), s);
+                if (mid + 1 < nz) s = __fma_rn(sgn * dB[em + t], __ldcg(z + em + n + t), s);
+                xs[p * n + t] = s;
+            }
+            __syncthreads();
+            const double r = product(nvis);
+            if (lead) z[em + row] = r;
+        }
+        cluster_sync_all();                                 // no store to a CTA that has left
+    } else if (yk2) {
+        __threadfence();
+        cluster_sync_all();
+        const int j0 = half ? mid + 1 : 0, j1 = half ? nz : mid + 1;
+        const size_t e0 = ((size_t)l0 + j0) * n;
+        const int ne = (j1 - j0) * n;
+        for (int e = rank * nth + tid; e < ne; e += csize * nth)
+            yk2[e0 + e] = y[e0 + e] + __ldcg(out + e0 + e) / R_ROS;
+    }
+}
+
 // ---------------------------------------------------------------------------
+namespace {
+// Launch configuration with clusters of cs CTAs.
+struct ClusterLaunch {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute at[1];
+    ClusterLaunch(int grid, int threads, size_t smem, int cs, cudaStream_t s) {
+        cfg.gridDim = dim3((unsigned)grid);
+        cfg.blockDim = dim3((unsigned)threads);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = s;
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = (unsigned)cs;
+        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+        cfg.attrs = at;
+        cfg.numAttrs = cs > 1 ? 1 : 0;
+    }
+};
+}  // namespace
+
 // CTAs per half-column.  While the half-columns do not fill the chip, sharing
 // each block between the CTAs of a cluster shortens the chain of its pivots
-// (one NCHO column: 9.8, 6.5, 5.0 and 4.4 ms with 1, 2, 4 and 8); the line
+// (one NCHO column: 9.8, 6.5, 5.0 and 4.2 ms with 1, 2, 4 and 8); the line
 // lies where every CTA still has an SM of its own, because beyond it the
-// shared FP64 units gain nothing (64 columns: 12.5, 12.4, 18.1 and 36.5 ms).
-static int lu64_cluster(const DevBatch &b, int n) {
-    if (n < kLu64MinCluster) return 1;
-    for (int cs = 8; cs > 1; cs /= 2)
-        if (2ll * b.ncols * cs <= b.nsm && lu64_smem(n, cs) <= 232448) return cs;
+// shared FP64 units gain nothing (64 columns: 12.2, 12.4, 18.1 and 36.5 ms),
+// and where the device holds all the clusters at once: an SM count that a
+// GPC does not divide into clusters leaves SMs over (nine columns: 18 clusters of eight
+// take two turns, 8.3 ms, 18 of four 4.7).
+static int cluster_size(const DevBatch &b, const int *limit, bool (*fits)(int, int), int n) {
+    for (int i = 2; i >= 0; --i)
+        if (2 * b.ncols <= limit[i] && 2ll * b.ncols * (2 << i) <= b.nsm && fits(n, 2 << i)) return 2 << i;
     return 1;
+}
+static bool lu64_fits(int n, int cs) { return n >= kLu64MinCluster && lu64_smem(n, cs) <= kMaxSmem; }
+// (the sweeps, one NCHO column, two solves: 0.89 ms with one CTA per half, 0.53 with eight)
+static bool sweep64_fits(int n, int cs) { return sweep64c_smem(n, cs) <= kMaxSmem; }
+
+template <class K>
+static int active_clusters(K *kernel, int threads, size_t smem, int cs) {
+    const ClusterLaunch L(cs, threads, smem, cs, nullptr);
+    int k = 0;
+    if (cudaOccupancyMaxActiveClusters(&k, kernel, &L.cfg) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    return k;
+}
+
+// Clusters of 2, 4 and 8 CTAs that the current device holds at once (after init_lu64).
+void cluster_limits(int n, int lu[3], int sweep[3]) {
+    for (int i = 0; i < 3; ++i) {
+        const int cs = 2 << i;
+        lu[i] = lu64_fits(n, cs) ? active_clusters(k_lu64<true, false>, lu64_threads(n, cs), lu64_smem(n, cs), cs) : 0;
+        sweep[i] = sweep64_fits(n, cs)
+                       ? active_clusters(k_sweep64c<true>, sweep64c_threads(n, cs), sweep64c_smem(n, cs), cs) : 0;
+    }
 }
 
 cudaError_t init_lu64(int n) {
-    size_t scl = 0;
-    for (int cs = 2; cs <= 8; cs *= 2)
-        if (n >= kLu64MinCluster && lu64_smem(n, cs) <= 232448 && lu64_smem(n, cs) > scl) scl = lu64_smem(n, cs);
-    cudaError_t e = raise_smem_limit(k_lu64<false>, lu64_smem(n, 1));
-    if (e == cudaSuccess && scl) e = raise_smem_limit(k_lu64<true>, scl);
-    const size_t ssw = sweep64_smem(n, 256, sweep64_nbuf(n, 1));
+    size_t scl = 0, ssc = 0;
+    for (int cs = 2; cs <= 8; cs *= 2) {
+        if (lu64_fits(n, cs) && lu64_smem(n, cs) > scl) scl = lu64_smem(n, cs);
+        if (sweep64_fits(n, cs) && sweep64c_smem(n, cs) > ssc) ssc = sweep64c_smem(n, cs);
+    }
+    cudaError_t e = raise_smem_limit(k_lu64<false, false>, lu64_smem(n, 1));
+    if (e == cudaSuccess && scl) e = raise_smem_limit(k_lu64<true, false>, scl);
+    const size_t ssw = sweep64_smem(n, sweep64_nbuf(n, 1));
     if (e == cudaSuccess) e = raise_smem_limit(k_sweep64<true>, ssw);
     if (e == cudaSuccess) e = raise_smem_limit(k_sweep64<false>, ssw);
+    if (e == cudaSuccess) e = raise_smem_limit(k_sweep64c<true>, ssc);
+    if (e == cudaSuccess) e = raise_smem_limit(k_sweep64c<false>, ssc);
     return e;
 }
 
 void launch_lu64(const DevNet &net, const DevBatch &b, const Work &w, cudaStream_t s) {
-    const int n = net.ni, cs = lu64_cluster(b, n);
+    const int n = net.ni, cs = cluster_size(b, b.ncl_lu, lu64_fits, n);
     reset_queue(b, s);
-    cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute at[1];
-    cfg.blockDim = dim3((unsigned)lu64_threads(n));
-    cfg.dynamicSmemBytes = lu64_smem(n, cs);
-    cfg.stream = s;
-    if (cs == 1) {
-        cfg.gridDim = dim3((unsigned)half_grid(b, VK_TUNE_LU64, 2));
-        cudaLaunchKernelEx(&cfg, k_lu64<false>, net, b, (const double *)w.jv, (const double *)w.dA,
-                           (const double *)w.dB, (const double *)w.dC, (const double *)w.dt, w.G,
-                           w.status, 1);
-        return;
-    }
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = (unsigned)cs;
-    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    cfg.gridDim = dim3((unsigned)(2 * b.ncols * cs));
-    cudaLaunchKernelEx(&cfg, k_lu64<true>, net, b, (const double *)w.jv, (const double *)w.dA,
-                       (const double *)w.dB, (const double *)w.dC, (const double *)w.dt, w.G, w.status,
-                       cs);
+    const ClusterLaunch L(cs == 1 ? half_grid(b, VK_TUNE_LU64, 2) : 2 * b.ncols * cs, lu64_threads(n, cs),
+                          lu64_smem(n, cs), cs, s);
+    cudaLaunchKernelEx(&L.cfg, cs == 1 ? k_lu64<false, false> : k_lu64<true, false>, net, b, (const double *)w.jv,
+                       (const double *)w.dA, (const double *)w.dB, (const double *)w.dC, (const double *)w.dt, w.G,
+                       w.status, cs, -1);
 }
 
-// CTAs of a sweep an SM should hold
-static int sweep64_ctas(const DevBatch &b) { return 2 * b.ncols <= b.nsm ? 1 : 2; }
+template <bool FWD>
+static void launch_sweep64(const DevNet &net, const DevBatch &b, const double *G, const double *dB, const double *dC,
+                           const double *rhs, double *z, double *x, const double *y, double *yk2, int *status,
+                           cudaStream_t s) {
+    const int n = net.ni, cs = cluster_size(b, b.ncl_sweep, sweep64_fits, n);
+    reset_queue(b, s);
+    if (cs > 1) {
+        const ClusterLaunch L(2 * b.ncols * cs, sweep64c_threads(n, cs), sweep64c_smem(n, cs), cs, s);
+        cudaLaunchKernelEx(&L.cfg, k_sweep64c<FWD>, n, block_stride64(n), b, G, dB, dC, 1.0, rhs, z, x, y, yk2,
+                           (const int *)status, cs, -1, 0);
+        return;
+    }
+    const int nbuf = sweep64_nbuf(n, 2 * b.ncols <= b.nsm ? 1 : 2);
+    k_sweep64<FWD><<<half_grid(b, VK_TUNE_SWEEP64, 2), sweep64_threads(n), sweep64_smem(n, nbuf), s>>>(
+        net, b, G, dB, dC, rhs, z, x, y, yk2, status, nbuf);
+}
 
 void launch_fwd64(const DevNet &net, const DevBatch &b, const double *G, const double *dB,
                   const double *dC, const double *rhs, double *z, int *status, cudaStream_t s) {
-    reset_queue(b, s);
-    const int nbuf = sweep64_nbuf(net.ni, sweep64_ctas(b));
-    k_sweep64<true><<<half_grid(b, VK_TUNE_SWEEP64, 2), 256, sweep64_smem(net.ni, 256, nbuf), s>>>(
-        net, b, G, dB, dC, rhs, z, nullptr, nullptr, nullptr, status, nbuf);
+    launch_sweep64<true>(net, b, G, dB, dC, rhs, z, nullptr, nullptr, nullptr, status, s);
 }
 
 void launch_back64(const DevNet &net, const DevBatch &b, const double *G, const double *dB,
                    const double *dC, double *z, double *x, const double *y, double *yk2, int *status,
                    cudaStream_t s) {
-    reset_queue(b, s);
-    const int nbuf = sweep64_nbuf(net.ni, sweep64_ctas(b));
-    k_sweep64<false><<<half_grid(b, VK_TUNE_SWEEP64, 2), 256, sweep64_smem(net.ni, 256, nbuf), s>>>(
-        net, b, G, dB, dC, nullptr, z, x, y, yk2, status, nbuf);
+    launch_sweep64<false>(net, b, G, dB, dC, nullptr, z, x, y, yk2, status, s);
+}
+
+// ---------------------------------------------------------------------------
+// One column whose blocks and couplings are given (vk_block_solve_noalloc).
+
+__global__ void k_solve64_words(int nz, int *words) {
+    words[0] = 0;                          // order
+    words[1] = 0;                          // col_off
+    words[2] = nz;                         // col_end
+    words[3] = 0;                          // status
+    for (int i = 4; i < kSolve64Words; ++i) words[i] = 0;       // queues of the two launches
+}
+
+cudaError_t init_solve64(int nmax) {
+    size_t scl = 0, ssc = 0;
+    for (int n = 1; n <= nmax; ++n) {
+        if (lu64_fits(n, 8) && lu64_smem(n, 8) > scl) scl = lu64_smem(n, 8);
+        if (sweep64c_smem(n, 8) > ssc) ssc = sweep64c_smem(n, 8);
+    }
+    cudaError_t e = raise_smem_limit(k_lu64<false, true>, lu64_smem(nmax, 1));
+    if (e == cudaSuccess) e = raise_smem_limit(k_lu64<true, true>, scl);
+    if (e == cudaSuccess) e = raise_smem_limit(k_sweep64c<true>, ssc);
+    if (e == cudaSuccess) e = raise_smem_limit(k_sweep64c<false>, ssc);
+    return e;
+}
+
+// G: nz n n doubles, z: nz n, words: kSolve64Words ints, words[3] the status.
+cudaError_t launch_solve64(int nz, int n, const double *D, const double *lo, const double *up, const double *rhs,
+                           double *x, double *G, double *z, int *words, int mid, cudaStream_t s) {
+    DevNet net = {};
+    net.ni = n;
+    DevBatch b = {};
+    b.ncols = 1;
+    b.L = nz;
+    b.order = words;
+    b.col_off = words + 1;
+    b.col_end = words + 2;
+    b.queue = reinterpret_cast<unsigned *>(words + 4);
+    int *status = words + 3;
+    k_solve64_words<<<1, 1, 0, s>>>(nz, words);
+    const int cl = lu64_fits(n, 8) ? 8 : 1;
+    const ClusterLaunch A(2 * cl, lu64_threads(n, cl), lu64_smem(n, cl), cl, s);
+    cudaError_t e = cudaLaunchKernelEx(&A.cfg, cl > 1 ? k_lu64<true, true> : k_lu64<false, true>, net, b, D,
+                                       (const double *)nullptr, up, lo, (const double *)nullptr, G, status, cl, mid);
+    if (e != cudaSuccess) return e;
+    const ClusterLaunch S(16, sweep64c_threads(n, 8), sweep64c_smem(n, 8), 8, s);
+    b.queue += 2;
+    e = cudaLaunchKernelEx(&S.cfg, k_sweep64c<true>, n, n * n, b, (const double *)G, up, lo, -1.0, rhs, z,
+                           (double *)nullptr, (const double *)nullptr, (double *)nullptr, (const int *)status, 8, mid, 1);
+    if (e != cudaSuccess) return e;
+    return cudaLaunchKernelEx(&S.cfg, k_sweep64c<false>, n, n * n, b, (const double *)G, up, lo, -1.0,
+                              (const double *)nullptr, z, x, (const double *)nullptr, (double *)nullptr,
+                              (const int *)status, 8, mid, 1);
 }
 
 }  // namespace vk

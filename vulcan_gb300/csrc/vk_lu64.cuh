@@ -39,11 +39,16 @@
 
 namespace vk {
 
-constexpr int kLu64BulkWarps = 6;      // enough to keep the FP64 unit busy from one CTA
 constexpr int kLu64MinCluster = 32;    // smallest block a cluster may share
 
 __host__ __device__ inline int lu64_prep_warps(int n) { return (n + 31) / 32; }
-__host__ __device__ inline int lu64_threads(int n) { return 32 * (lu64_prep_warps(n) + kLu64BulkWarps); }
+// Bulk warps of a CTA that has a block to itself, as many on each of the SM's
+// four schedulers (512 NCHO columns: 6, 8, 10, 12 and 14 warps 49.4, 49.5, 47.1,
+// 46.0 and 47.4 ms), and of a cluster's (one column: 6, 7, 12 warps 4.41, 4.21
+// and 4.17 ms, seven of 89 species 8.46, 8.16 and 8.49).
+__host__ __device__ inline int lu64_threads(int n, int csize) {
+    return 32 * (lu64_prep_warps(n) + (csize > 1 ? 7 : 12));
+}
 // doubles of a message: 1/pivot, pivot row, n multipliers, to a multiple of 16 bytes
 __host__ __device__ inline int lu64_msg(int n) { return (n + 3) & ~1; }
 // first column of rank c's slice
