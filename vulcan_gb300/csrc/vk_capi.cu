@@ -77,7 +77,7 @@ struct vk_handle {
     int cps = 0;                        // VK_CTAS_PER_SM override (0: kernel defaults)
     int cps_k[VK_TUNE_N] = {0, 0, 0, 0}; // vk_set_launch: CTAs per SM per kernel
     int lu32_tiling = -1;               // vk_set_launch: k_lu32 variant (-1: by ni)
-    int occ_rates = 0, occ_prep = 0;    // resident CTAs per SM of k_rates / k_prep32
+    int occ_rates[3] = {}, occ_prep = 0;    // resident CTAs per SM of k_rates (tiles of 1, 2, 4 layers) / k_prep32
     double *d_k = nullptr, *d_atm = nullptr, *d_Dzz = nullptr, *d_spf = nullptr;
     vk::Work w{};
     // batched-run state
@@ -123,7 +123,7 @@ struct vk_handle {
         b.cps = cps;
         for (int i = 0; i < VK_TUNE_N; ++i) b.cps_k[i] = cps_k[i];
         b.lu32_tiling = lu32_tiling;
-        b.grid_rates = nsm * occ_rates;
+        for (int i = 0; i < 3; ++i) b.grid_rates[i] = nsm * occ_rates[i];
         b.grid_prep = nsm * occ_prep;
         return b;
     }
@@ -372,7 +372,7 @@ extern "C" int vk_create(const vk_network *net, int max_cols, int max_layers, in
     TRY(vk::init_prep32(h->net()) == cudaSuccess && vk::init_lu32(h->ni) == cudaSuccess
             ? VK_OK : fail(h, VK_ECUDA, "cudaFuncSetAttribute (FP32 LU) failed"));
     vk::cluster_limits(h->ni, h->ncl_lu, h->ncl_sweep);
-    h->occ_rates = vk::rates_blocks_per_sm(h->net());
+    vk::rates_blocks_per_sm(h->net(), h->occ_rates);
     h->occ_prep = vk::prep_blocks_per_sm(h->net());
     cudaGetLastError();                 // an occupancy query that failed leaves one CTA per layer
     // per-column run state (small); the history ring is sized at the first vk_run
@@ -636,7 +636,7 @@ static void enqueue_solves64(vk_handle *h, const DevNet &net, const DevBatch &b,
     vk::Work &w = h->w;
     vk::launch_fwd64(net, b, w.G, w.dB, w.dC, w.f, w.z, w.status, s);
     vk::launch_back64(net, b, w.G, w.dB, w.dC, w.z, w.k1, w.y, w.yk2, w.status, s);
-    vk::launch_rates(net, b, w.yk2, w.f, nullptr, nullptr, nullptr, nullptr, w.k1, w.dt, w.geo, flags, false, s);
+    vk::launch_rates(net, b, w.yk2, w.f, nullptr, nullptr, nullptr, nullptr, w.k1, w.dt, w.geo, flags, false, false, s);
     vk::launch_fwd64(net, b, w.G, w.dB, w.dC, w.f, w.z, w.status, s);
     vk::launch_back64(net, b, w.G, w.dB, w.dC, w.z, w.k2, w.y, nullptr, w.status, s);
 }
@@ -648,7 +648,7 @@ static void enqueue_attempt_kernels(vk_handle *h, const DevNet &net, const DevBa
     vk::Work &w = h->w;
     cudaStream_t s = h->stream;
     if (timed) cudaEventRecord(h->ev[0], s);
-    vk::launch_rates(net, b, w.y, w.f, w.jv, w.dA, w.dB, w.dC, nullptr, w.dt, w.geo, flags, true, s);
+    vk::launch_rates(net, b, w.y, w.f, w.jv, w.dA, w.dB, w.dC, nullptr, w.dt, w.geo, flags, true, false, s);
     if (timed) cudaEventRecord(h->ev[1], s);
     if (h->precision == VK_PREC_FP64) {
         vk::launch_lu64(net, b, w, s);
@@ -677,7 +677,7 @@ static void enqueue_attempt_kernels(vk_handle *h, const DevNet &net, const DevBa
         vk::launch_lu32(net, b32, w, s);
         if (timed) cudaEventRecord(h->ev[2], s);
         vk::launch_refine(net, b32, w, w.f, w.k1, w.y, w.yk2, h->max_refine, h->refine_tol, s);
-        vk::launch_rates(net, b32, w.yk2, w.f2, nullptr, nullptr, nullptr, nullptr, w.k1, w.dt, w.geo, flags, false, s);
+        vk::launch_rates(net, b32, w.yk2, w.f2, nullptr, nullptr, nullptr, nullptr, w.k1, w.dt, w.geo, flags, false, false, s);
         vk::launch_refine(net, b32, w, w.f2, w.k2, w.y, nullptr, h->max_refine, h->refine_tol, s);
         cudaStreamWaitEvent(s, h->ev_join, 0);
         // columns whose refinement failed: FP64 after the others (their f(y)
@@ -754,7 +754,7 @@ extern "C" int vk_rhs(vk_handle *h, const double *y, int flags, double *f) {
     }
     ensure_geometry(h, flags);
     vk::launch_rates(h->net(), h->batch(), yd, h->w.f2, h->w.jv, h->w.dA, h->w.dB, h->w.dC, nullptr,
-                     h->w.dt, h->w.geo, flags, false, h->stream);
+                     h->w.dt, h->w.geo, flags, false, false, h->stream);
     VK_CUDA(h, cudaGetLastError());
     VK_CUDA(h, cudaMemcpyAsync(f, h->w.f2, bytes, cudaMemcpyDeviceToHost, h->stream));
     VK_CUDA(h, cudaStreamSynchronize(h->stream));

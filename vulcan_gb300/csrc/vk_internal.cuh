@@ -127,9 +127,9 @@ struct DevBatch {
                                // (0: each kernel's own default)
     int cps_k[VK_TUNE_N];      // per-kernel setting of vk_set_launch (0: cps)
     int lu32_tiling;           // k_lu32 variant (-1: by ni)
-    int grid_rates, grid_prep; // CTAs of the per-layer kernels k_rates / k_prep32:
-                               // all of them resident at once, each striding over
-                               // the layers (0: one CTA per layer)
+    int grid_rates[3];         // CTAs of k_rates with tiles of 1, 2 and 4 layers: all of
+                               // them resident at once, each striding over the tiles
+    int grid_prep;             // the same of k_prep32, over the layers (0: one CTA each)
 };
 
 // Grid of a per-layer kernel whose CTAs stride over the layers: as many CTAs
@@ -241,7 +241,7 @@ struct Work {                  // per-handle device work buffers
 
 void launch_rates(const DevNet &net, const DevBatch &b, const double *y, double *f,
                   double *jv, double *dA, double *dB, double *dC, const double *k1,
-                  const double *dt, const double *geo, int flags, bool with_jac, cudaStream_t s);
+                  const double *dt, const double *geo, int flags, bool with_jac, bool chem_only, cudaStream_t s);
 void launch_geometry(const DevNet &net, const DevBatch &b, double *geo, int flags, cudaStream_t s);
 cudaError_t init_lu64(int n);
 void cluster_limits(int n, int lu[3], int sweep[3]);
@@ -274,7 +274,7 @@ cudaError_t init_prep32(const DevNet &net);
 cudaError_t init_lu32(int n);
 // Resident CTAs per SM of the per-layer kernels for a network (0: unknown);
 // call after the init_* functions have raised their shared-memory limits.
-int rates_blocks_per_sm(const DevNet &net);
+void rates_blocks_per_sm(const DevNet &net, int occ[3]);
 int prep_blocks_per_sm(const DevNet &net);
 void launch_prep32(const DevNet &net, const DevBatch &b, const Work &w, cudaStream_t s);
 void launch_lu32(const DevNet &net, const DevBatch &b, const Work &w, cudaStream_t s);
