@@ -383,17 +383,21 @@ k_sweep64(DevNet net, DevBatch b, const double *G, const double *__restrict__ dB
 // --- a cluster per half-column: CTA c has the rows [c n / cs, (c + 1) n / cs),
 // eight lanes each (one part), whose blocks a lane copies itself, kSweepAhead
 // visits ahead (its own copies need no barrier).  The eight lanes
-// send the row of the next input to one CTA each; one cluster barrier a visit.
-// Results are kept in shared memory for kSweepHist visits: a store to global
-// memory before the barrier would have to be acknowledged there.
+// send the row of the next input to one CTA each, tagged with the visit: a lane
+// waits for the entries it reads, and no barrier is needed.  (Two input buffers
+// are enough: a row is sent when all entries of the visit before have been
+// read by its warp, and every CTA needs all rows to go on.)
+// Results are kept in shared memory for kSweepHist visits: waiting stores to
+// global memory would hold up the ones to the cluster.
 // Bound by the chain of a visit: n / 8 dependent FMAs, three exchanges and the
-// barrier. 
-// Two solves of one NCHO column of 150 layers 0.89 -> 0.53 ms (one CTA per half before).
+// way to the other CTAs.
+// Two solves of one NCHO column of 150 layers: 0.89 ms with one CTA per half,
+// 0.53 with a cluster barrier a visit, 0.49.
 constexpr int kSweepAhead = 4;
 constexpr int kSweepHist = 32;          // visits whose results wait in shared memory
 __host__ __device__ inline int sweep64c_threads(int n, int cs) { return (8 * lu64_slice_max(n, cs) + 31) / 32 * 32; }
 __host__ __device__ inline size_t sweep64c_smem(int n, int cs) {
-    return (size_t)(kSweepAhead * ((n + 7) / 8 + 2) * sweep64c_threads(n, cs) + 2 * n +
+    return (size_t)(kSweepAhead * ((n + 7) / 8 + 2) * sweep64c_threads(n, cs) + 4 * n +
                     kSweepHist * lu64_slice_max(n, cs)) * sizeof(double);
 }
 
@@ -404,15 +408,14 @@ template <bool FWD>
 __global__ void __launch_bounds__(640)
 k_sweep64c(int n, int gst, DevBatch b, const double *G, const double *__restrict__ dB,
            const double *__restrict__ dC, double sgn, const double *__restrict__ rhs, double *z, double *out,
-           const double *__restrict__ y, double *__restrict__ yk2, const int *__restrict__ status, int csize,
-           int mid1, int skip) {
+           const double *__restrict__ y, double *__restrict__ yk2, int *status, int csize, int mid1, int skip) {
     extern __shared__ __align__(16) double smc[];
-    __shared__ int s_unit;
+    __shared__ int s_unit, s_dead;
     const int tid = threadIdx.x, nth = blockDim.x, K = (n + 7) / 8;
     double *ring = smc;                                     // [ahead][K][nth] each lane's part of its row
     double *vec = ring + kSweepAhead * K * nth;             // [ahead][2][nth] coupling, rhs or z
-    double *xs = vec + kSweepAhead * 2 * nth;               // [2][n] inputs of two visits
-    double *hist = xs + 2 * n;                              // [kSweepHist][rows] results
+    ulonglong2 *xs = reinterpret_cast<ulonglong2 *>(vec + kSweepAhead * 2 * nth);   // [2][n] tagged inputs of two visits
+    double *hist = reinterpret_cast<double *>(xs + 2 * n);  // [kSweepHist][rows] results
     const int rank = (int)cluster_rank(), u = (int)blockIdx.x / csize;
     const int r0 = lu64_slice(n, csize, rank), r1 = lu64_slice(n, csize, rank + 1);
     const int row = r0 + (tid >> 3), part = tid & 7;
@@ -443,38 +446,49 @@ k_sweep64c(int n, int gst, DevBatch b, const double *G, const double *__restrict
         cp_async_commit();
     };
     for (int v = 0; v < kSweepAhead - 1; ++v) fetch(v);
+    if (tid == 0) s_dead = 0;
+    for (int t = tid; t < n; t += nth) xs[n + t] = make_ulonglong2(0, 0);
     if (FWD) {
         if (nvis > 0)
-            for (int t = tid; t < n; t += nth) xs[t] = rhs[e1 + t];
+            for (int t = tid; t < n; t += nth) xs[t] = tagged(rhs[e1 + t], 1);
     } else {
         const size_t em = ((size_t)l0 + mid) * n;
         if (nvis > 0)
-            for (int t = tid; t < n; t += nth) xs[t] = (sgn * cpl[e1 + t]) * z[em + t];
+            for (int t = tid; t < n; t += nth) xs[t] = tagged((sgn * cpl[e1 + t]) * z[em + t], 1);
         if (half == 0 && lead) out[em + row] = z[em + row];
     }
-    __syncthreads();
-    int p = 0;
+    const uint32_t xs0 = smem_u32(xs);
     auto product = [&](int v) {
-        const double *g = ring + (v % kSweepAhead) * K * nth + tid, *xin = xs + p * n;
+        const double *g = ring + (v % kSweepAhead) * K * nth + tid;
+        const uint32_t xin = xs0 + (uint32_t)((v & 1) * n) * 16u;
+        const unsigned tag = (unsigned)v + 1;
         double a = 0.0;
-        if (rowt) {
-            int i = 0, q = part;
-            for (; q + 24 < n; q += 32, i += 4) {
-                const double g0 = g[i * nth], g1 = g[(i + 1) * nth], g2 = g[(i + 2) * nth], g3 = g[(i + 3) * nth];
-                const double x0 = xin[q], x1 = xin[q + 8], x2 = xin[q + 16], x3 = xin[q + 24];
-                a = __fma_rn(g0, x0, a);
-                a = __fma_rn(g1, x1, a);
-                a = __fma_rn(g2, x2, a);
-                a = __fma_rn(g3, x3, a);
+        if (rowt)
+            for (int i = 0, q = part; q < n; q += 96, i += 12) {    // twelve entries at a time
+                double x[12];
+#pragma unroll
+                for (int u = 0; u < 12; ++u) x[u] = 0.0;
+                for (int tries = 0;; ++tries) {
+                    bool ok = true;
+#pragma unroll
+                    for (int u = 0; u < 12; ++u)
+                        if (q + 8 * u < n) ok &= get_tagged(xin + (uint32_t)(q + 8 * u) * 16u, x[u], tag);
+                    if (ok) break;
+                    if ((tries & 255) == 255 && (tries >= kMbarSpin || *(volatile int *)&s_dead)) {
+                        *(volatile int *)&s_dead = 1;
+                        break;
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < 12; ++u)
+                    if (q + 8 * u < n) a = __fma_rn(g[(i + u) * nth], x[u], a);
             }
-            for (; q < n; q += 8, ++i) a = __fma_rn(g[i * nth], xin[q], a);
-        }
         __syncwarp();
         a += __shfl_xor_sync(0xffffffffu, a, 4);
         a += __shfl_xor_sync(0xffffffffu, a, 1);
         return a + __shfl_xor_sync(0xffffffffu, a, 2);
     };
-    const uint32_t peer = part < csize ? cluster_addr(smem_u32(xs), (uint32_t)part) : 0u;
+    const uint32_t peer = part < csize ? cluster_addr(xs0, (uint32_t)part) : 0u;
     cluster_sync_all();                                     // every CTA of the cluster runs
     for (int v = 0; v < nvis; ++v) {
         cp_async_wait<kSweepAhead - 2>();
@@ -484,12 +498,10 @@ k_sweep64c(int n, int gst, DevBatch b, const double *G, const double *__restrict
             if (!FWD) r += s[nth];
             if (v + 1 < nvis && part < csize) {
                 const double f = sgn * s[0], xn = FWD ? __fma_rn(f, r, s[nth]) : f * r;
-                asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(peer + (uint32_t)((p ^ 1) * n + row) * 8u), "d"(xn)
-                             : "memory");
+                put_tagged(peer + (uint32_t)(((v + 1) & 1) * n + row) * 16u, xn, (unsigned)v + 2);
             }
             if (part == 0) hist[(v % kSweepHist) * (r1 - r0) + row - r0] = r;
         }
-        asm volatile("barrier.cluster.arrive.release;" ::: "memory");
         fetch(v + kSweepAhead - 1);
         if (v + 1 == nvis || (v + 1) % kSweepHist == 0) {
             __syncwarp();
@@ -499,8 +511,6 @@ k_sweep64c(int n, int gst, DevBatch b, const double *G, const double *__restrict
                     (FWD ? z : out)[e1 + es * t + row] = hist[(t - v0) * (r1 - r0) + row - r0];
             __syncwarp();
         }
-        asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
-        p ^= 1;
     }
     cp_async_wait<0>();
     if (FWD) {
@@ -510,13 +520,12 @@ k_sweep64c(int n, int gst, DevBatch b, const double *G, const double *__restrict
                 double s = rhs[em + t];
                 if (mid > 0) s = __fma_rn(sgn * dC[em + t], __ldcg(z + em - n + t), s);
                 if (mid + 1 < nz) s = __fma_rn(sgn * dB[em + t], __ldcg(z + em + n + t), s);
-                xs[p * n + t] = s;
+                xs[(nvis & 1) * n + t] = tagged(s, (unsigned)nvis + 1);
             }
             __syncthreads();
             const double r = product(nvis);
             if (lead) z[em + row] = r;
         }
-        cluster_sync_all();                                 // no store to a CTA that has left
     } else if (yk2) {
         __threadfence();
         cluster_sync_all();
@@ -526,6 +535,8 @@ k_sweep64c(int n, int gst, DevBatch b, const double *G, const double *__restrict
         for (int e = rank * nth + tid; e < ne; e += csize * nth)
             yk2[e0 + e] = y[e0 + e] + __ldcg(out + e0 + e) / R_ROS;
     }
+    cluster_sync_all();                                     // no store to a CTA that has left
+    if (tid == 0 && s_dead) atomicExch(&status[c], VK_ETIMEOUT);
 }
 
 // ---------------------------------------------------------------------------
@@ -562,7 +573,7 @@ static int cluster_size(const DevBatch &b, const int *limit, bool (*fits)(int, i
     return 1;
 }
 static bool lu64_fits(int n, int cs) { return n >= kLu64MinCluster && lu64_smem(n, cs) <= kMaxSmem; }
-// (the sweeps, one NCHO column, two solves: 0.89 ms with one CTA per half, 0.53 with eight)
+// (the sweeps, one NCHO column, two solves: 0.89 ms with one CTA per half, 0.49 with eight)
 static bool sweep64_fits(int n, int cs) { return sweep64c_smem(n, cs) <= kMaxSmem; }
 
 template <class K>
@@ -621,7 +632,7 @@ static void launch_sweep64(const DevNet &net, const DevBatch &b, const double *G
     if (cs > 1) {
         const ClusterLaunch L(2 * b.ncols * cs, sweep64c_threads(n, cs), sweep64c_smem(n, cs), cs, s);
         cudaLaunchKernelEx(&L.cfg, k_sweep64c<FWD>, n, block_stride64(n), b, G, dB, dC, 1.0, rhs, z, x, y, yk2,
-                           (const int *)status, cs, -1, 0);
+                           status, cs, -1, 0);
         return;
     }
     const int nbuf = sweep64_nbuf(n, 2 * b.ncols <= b.nsm ? 1 : 2);
@@ -686,11 +697,11 @@ cudaError_t launch_solve64(int nz, int n, const double *D, const double *lo, con
     const ClusterLaunch S(16, sweep64c_threads(n, 8), sweep64c_smem(n, 8), 8, s);
     b.queue += 2;
     e = cudaLaunchKernelEx(&S.cfg, k_sweep64c<true>, n, n * n, b, (const double *)G, up, lo, -1.0, rhs, z,
-                           (double *)nullptr, (const double *)nullptr, (double *)nullptr, (const int *)status, 8, mid, 1);
+                           (double *)nullptr, (const double *)nullptr, (double *)nullptr, status, 8, mid, 1);
     if (e != cudaSuccess) return e;
     return cudaLaunchKernelEx(&S.cfg, k_sweep64c<false>, n, n * n, b, (const double *)G, up, lo, -1.0,
                               (const double *)nullptr, z, x, (const double *)nullptr, (double *)nullptr,
-                              (const int *)status, 8, mid, 1);
+                              status, 8, mid, 1);
 }
 
 }  // namespace vk

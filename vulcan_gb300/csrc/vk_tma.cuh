@@ -56,6 +56,24 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
+// A double and a tag in two 64-bit words, each of them single-copy atomic: a
+// reader of its shared memory that finds the tag in both has the value, and
+// the writer in another CTA of the cluster needs no fence.
+__device__ __forceinline__ ulonglong2 tagged(double v, unsigned tag) {
+    const unsigned long long u = (unsigned long long)__double_as_longlong(v), t = (unsigned long long)tag << 32;
+    return make_ulonglong2((u & 0xffffffffull) | t, (u >> 32) | t);
+}
+__device__ __forceinline__ void put_tagged(uint32_t cluster_smem, double v, unsigned tag) {
+    const ulonglong2 w = tagged(v, tag);
+    asm volatile("st.volatile.shared::cluster.v2.b64 [%0], {%1, %2};" ::"r"(cluster_smem), "l"(w.x), "l"(w.y) : "memory");
+}
+__device__ __forceinline__ bool get_tagged(uint32_t smem, double &v, unsigned tag) {
+    unsigned long long a, b;
+    asm volatile("ld.volatile.shared::cta.v2.b64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "r"(smem) : "memory");
+    v = __longlong_as_double((long long)((a & 0xffffffffull) | (b << 32)));
+    return (unsigned)(a >> 32) == tag && (unsigned)(b >> 32) == tag;
+}
+
 // Padded stride (floats) of an n x n FP32 block so every block starts on 16 bytes.
 __host__ __device__ __forceinline__ int block_stride32(int n) { return (n * n + 3) & ~3; }
 
