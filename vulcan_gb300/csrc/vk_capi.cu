@@ -64,6 +64,10 @@ struct vk_handle {
     double *d_crossT = nullptr, *d_wcrossJT = nullptr;
     int tcap_abs = 0, tcap_ch = 0;      // table rows allocated
     int *d_kkind = nullptr, *d_krev = nullptr;   // rate-constant parameters (vk_set_rate_params)
+    int *d_rt_off = nullptr;            // and their distinct exponents
+    double *d_rt_val = nullptr;
+    int4 *d_rt_idx = nullptr;
+    vk::RateTab rate_tab = {};
     double *d_kpar = nullptr, *d_nasa9 = nullptr;
     int *d_capk = nullptr;              // low-temperature caps (vk_set_rate_caps)
     double *d_capT = nullptr, *d_capp = nullptr;
@@ -884,6 +888,52 @@ extern "C" int vk_get_counters(vk_handle *h, int *counters) {
     return VK_OK;
 }
 
+// The distinct exponents of the pairs' rate constants, in chunks of consecutive
+// pairs with at most kRateTabCap of them (vk_rates_k.cu).
+static void rate_table(int npair, const int *kind, const double *params, std::vector<int> &pair_off,
+                       std::vector<int> &tab_off, std::vector<double> &val, std::vector<int4> &idx,
+                       std::vector<int> &special) {
+    std::vector<double> B, C;              // of the open chunk
+    int sp[7] = {};
+    idx.assign(npair, make_int4(0, 0, 0, 0));
+    pair_off.assign(1, 0);
+    tab_off.assign(1, 0);
+    auto find = [](std::vector<double> &v, double x) {
+        size_t i = 0;
+        while (i < v.size() && std::memcmp(&v[i], &x, sizeof x) != 0) ++i;
+        if (i == v.size()) v.push_back(x);
+        return (int)i;
+    };
+    auto close = [&](int p) {
+        const int nB = (int)B.size();      // C's entries follow B's
+        for (int q = pair_off.back(); q < p; ++q) { idx[q].y += nB; idx[q].w += nB; }
+        for (int i = 0; i < 7; ++i) special.push_back(i < 3 ? sp[i] : sp[i] + nB);
+        val.insert(val.end(), B.begin(), B.end());
+        tab_off.push_back((int)val.size());
+        val.insert(val.end(), C.begin(), C.end());
+        tab_off.push_back((int)val.size());
+        pair_off.push_back(p);
+        B.clear();
+        C.clear();
+        std::fill(sp, sp + 7, 0);
+    };
+    for (int p = 0; p < npair; ++p) {
+        if ((int)(B.size() + C.size()) + 7 > vk::kRateTabCap) close(p);
+        const double *pp = params + (size_t)p * 6;
+        if (kind[p] == VK_K_ARRHENIUS || kind[p] == VK_K_FALLOFF) {
+            idx[p].x = find(B, pp[1]);
+            idx[p].y = find(C, pp[2]);
+        }
+        if (kind[p] == VK_K_FALLOFF) {
+            idx[p].z = find(B, pp[4]);
+            idx[p].w = find(C, pp[5]);
+        }
+        if (kind[p] == VK_K_SPECIAL_OH_CH3)
+            for (int i = 0; i < 7; ++i) sp[i] = find(i < 3 ? B : C, vk::kRateSpecial[i]);
+    }
+    close(npair);
+}
+
 extern "C" int vk_set_rate_params(vk_handle *h, const int *kind, const int *rev, const double *params,
                                   const double *nasa9) {
     if (!h) return fail(h, VK_EINVAL, "handle is NULL");
@@ -896,11 +946,37 @@ extern "C" int vk_set_rate_params(vk_handle *h, const int *kind, const int *rev,
         if (!rc) rc = dalloc(h, &h->d_krev, h->npair);
         if (!rc) rc = dalloc(h, &h->d_kpar, (size_t)h->npair * 6);
         if (!rc) rc = dalloc(h, &h->d_nasa9, (size_t)h->ni * 20);
+        if (!rc) rc = dalloc(h, &h->d_rt_off, (size_t)10 * h->npair + 20);
+        if (!rc) rc = dalloc(h, &h->d_rt_val, (size_t)11 * h->npair + 11);
+        if (!rc) rc = dalloc(h, &h->d_rt_idx, (size_t)h->npair);
         if (rc) {                          // the handle frees what was allocated
             h->d_kkind = nullptr;
             return rc;
         }
     }
+    std::vector<int> pair_off, tab_off, special, off;
+    std::vector<double> val;
+    std::vector<int4> idx;
+    try {
+        rate_table(h->npair, kind, params, pair_off, tab_off, val, idx, special);
+        off = pair_off;
+        off.insert(off.end(), tab_off.begin(), tab_off.end());
+        off.insert(off.end(), special.begin(), special.end());
+    } catch (const std::bad_alloc &) {
+        return fail(h, VK_ENOMEM, "out of host memory");
+    }
+    vk::RateTab &rt = h->rate_tab;
+    rt.nchunk = (int)pair_off.size() - 1;
+    rt.cap = 0;
+    for (int c = 0; c < rt.nchunk; ++c) rt.cap = std::max(rt.cap, tab_off[2 * c + 2] - tab_off[2 * c]);
+    rt.pair_off = h->d_rt_off;
+    rt.tab_off = h->d_rt_off + pair_off.size();
+    rt.special = rt.tab_off + tab_off.size();
+    rt.val = h->d_rt_val;
+    rt.idx = h->d_rt_idx;
+    VK_CUDA(h, cudaMemcpy(h->d_rt_off, off.data(), off.size() * sizeof(int), cudaMemcpyHostToDevice));
+    VK_CUDA(h, cudaMemcpy(h->d_rt_val, val.data(), val.size() * sizeof(double), cudaMemcpyHostToDevice));
+    VK_CUDA(h, cudaMemcpy(h->d_rt_idx, idx.data(), idx.size() * sizeof(int4), cudaMemcpyHostToDevice));
     VK_CUDA(h, cudaMemcpy(h->d_kkind, kind, h->npair * sizeof(int), cudaMemcpyHostToDevice));
     VK_CUDA(h, cudaMemcpy(h->d_krev, rev, h->npair * sizeof(int), cudaMemcpyHostToDevice));
     VK_CUDA(h, cudaMemcpy(h->d_kpar, params, (size_t)h->npair * 6 * sizeof(double), cudaMemcpyHostToDevice));
@@ -1137,7 +1213,7 @@ extern "C" int vk_compute_k(vk_handle *h) {
     int rc = need_batch(h);
     if (rc) return rc;
     if (!h->d_kkind) return fail(h, VK_EINVAL, "no rate parameters (call vk_set_rate_params)");
-    vk::launch_rate_consts(h->net(), h->batch(), h->d_kkind, h->d_krev,
+    vk::launch_rate_consts(h->net(), h->batch(), h->rate_tab, h->d_kkind, h->d_krev,
                            h->caps_on ? h->d_capk : nullptr, h->d_capT, h->d_capp, h->d_kpar,
                            h->d_nasa9, h->d_k, h->stream);
     VK_CUDA(h, cudaGetLastError());

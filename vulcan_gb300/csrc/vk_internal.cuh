@@ -261,7 +261,19 @@ void launch_stage(const DevNet &net, const DevBatch &b, const Work &w, int flags
 void launch_refine(const DevNet &net, const DevBatch &b, const Work &w, const double *rhs,
                    double *x, const double *yscale, double *yk2, int max_sweeps, double tol,
                    cudaStream_t s);
-void launch_rate_consts(const DevNet &net, const DevBatch &b, const int *kind, const int *rev,
+// Distinct exponents of the pairs' rate constants, in chunks of consecutive pairs
+// (rate_table): T^B for val[tab_off[2c] .. tab_off[2c+1]), exp(-C/T) up to tab_off[2c+2].
+constexpr int kRateTabCap = 1024;        // entries of a chunk
+constexpr double kRateSpecial[7] = {-9.88, -6.25, -0.018, 7544., 1433., -16.74, 4531.};
+struct RateTab {
+    int nchunk, cap;                     // chunks; most entries of one
+    const int *pair_off;                 // [nchunk + 1] first pair
+    const int *tab_off;                  // [2 nchunk + 1]
+    const double *val;
+    const int4 *idx;                     // [npair] entries of (B, C) and of the second (B, C), in the chunk
+    const int *special;                  // [nchunk][7] entries of kRateSpecial, where a pair needs them
+};
+void launch_rate_consts(const DevNet &net, const DevBatch &b, const RateTab &rt, const int *kind, const int *rev,
                         const int *cap_kind, const double *cap_T, const double *cap_params,
                         const double *params, const double *nasa9, double *k, cudaStream_t s);
 void launch_photo(const DevNet &net, const DevBatch &b, const PhotoDev &ph, const double *y,
