@@ -23,7 +23,7 @@
 // plenty.  A blocked elimination on the tensor cores shortens the updates, not
 // that chain.  With k_prep32, 69 species: 512 columns 11.0 -> 6.3 ms, 64
 // columns 7.0 -> 2.95 ms (tcgen05 rank-16 panels before); 150 species, 48
-// columns: 54 -> 13.2 ms (a one-sided register elimination with the block
+// columns: 54 -> 13.6 ms (a one-sided register elimination with the block
 // spread by 8 x 19 tiles before).
 //
 // Reference: the banded LU of the Ros2 LHS, op.py:2913-2929 (solve_banded on
@@ -44,12 +44,12 @@ constexpr int kSlot = 168;               // multipliers by row, then pivot row, 
 struct Lu32Smem {                        // float offsets
     int Gs, D, ms, row, alpha, beta, srow, perm, kinv, end;
 };
-__host__ __device__ inline Lu32Smem lu32_layout(int n, int cw, int w, bool dbuf) {
+__host__ __device__ inline Lu32Smem lu32_layout(int n, int cw, int w) {
     const int nn4 = block_stride32(n);
     Lu32Smem s;
     int o = 0;
     s.Gs = o;    o += nn4;
-    s.D = o;     o += dbuf ? nn4 : 0;
+    s.D = o;     o += nn4;
     s.ms = o;    o += 2 * kSlot;
     s.row = o;   o += w * ((cw + 3) & ~3);
     s.alpha = o; o += n;
@@ -63,9 +63,8 @@ __host__ __device__ inline Lu32Smem lu32_layout(int n, int cw, int w, bool dbuf)
 
 }  // namespace
 
-// DBUF: the next layer's block is copied to shared memory while this one is
-// inverted (n <= 128); otherwise it is read when its turn comes.
-template <int RA, int CW, int W, bool DBUF>
+// The next layer's block is copied to shared memory while this one is inverted.
+template <int RA, int CW, int W>
 __global__ void __launch_bounds__(32 * W, W == 4 ? (RA * CW <= 54 ? 4 : 3) : 1)
 k_lu32(DevNet net, DevBatch b, const float *__restrict__ D32, const double *__restrict__ dB,
        const double *__restrict__ dC, const double *__restrict__ rsc, const double *__restrict__ csc,
@@ -75,7 +74,7 @@ k_lu32(DevNet net, DevBatch b, const float *__restrict__ D32, const double *__re
     constexpr int CP = (CW + 3) & ~3;
     constexpr int NTH = 32 * W;
     const int n = net.ni, NNP = block_stride32(n);
-    const Lu32Smem L = lu32_layout(n, CW, W, DBUF);
+    const Lu32Smem L = lu32_layout(n, CW, W);
     float *Gs = smf + L.Gs, *Db = smf + L.D, *ms = smf + L.ms, *alpha = smf + L.alpha, *beta = smf + L.beta;
     float *srow = smf + L.srow;
     int *perm = reinterpret_cast<int *>(smf + L.perm), *kinv = reinterpret_cast<int *>(smf + L.kinv);
@@ -272,7 +271,7 @@ k_lu32(DevNet net, DevBatch b, const float *__restrict__ D32, const double *__re
             }
         };
         if (tid == 0) s_stat = 0;
-        if (DBUF && cnt > 0) prefetch(layer(0));
+        if (cnt > 0) prefetch(layer(0));
         for (int t = 0; t < cnt; ++t) {
             const size_t l = layer(t), lp = half ? l + 1 : l - 1;
             for (int q = tid; q < n && t > 0; q += NTH) {
@@ -280,11 +279,11 @@ k_lu32(DevNet net, DevBatch b, const float *__restrict__ D32, const double *__re
                 alpha[q] = (float)(rsc[l * n + q] * cr * csc[lp * n + q]);
                 beta[q] = (float)(rsc[lp * n + q] * cc * csc[l * n + q]);
             }
-            if (DBUF) asm volatile("cp.async.wait_group 0;" ::: "memory");
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
             __syncthreads();
-            load(DBUF ? Db : D32 + l * NNP, t > 0);
+            load(Db, t > 0);
             __syncthreads();                              // Db and Gs are free
-            if (DBUF && t + 1 < cnt) prefetch(layer(t + 1));
+            if (t + 1 < cnt) prefetch(layer(t + 1));
             invert();
             store(l);
         }
@@ -322,18 +321,18 @@ k_lu32(DevNet net, DevBatch b, const float *__restrict__ D32, const double *__re
 }
 
 // ---------------------------------------------------------------------------
-// The tilings: rows per lane, columns per warp, warps, block prefetched; the
+// The tilings: rows per lane, columns per warp, warps; the
 // smallest that covers the block (n <= 32 RA and n <= CW W) has the least work.
 #define VK_LU32_TILINGS(X) \
-    X(2, 12, 4, true) X(2, 16, 4, true) X(3, 18, 4, true) X(3, 24, 4, true) X(4, 16, 8, true) X(5, 20, 8, false)
+    X(2, 12, 4) X(2, 16, 4) X(3, 18, 4) X(3, 24, 4) X(4, 16, 8) X(5, 10, 16)
 static const int kTileCap[6] = {48, 64, 72, 96, 128, 160};
-static const int kTileCW[6] = {12, 16, 18, 24, 16, 20}, kTileW[6] = {4, 4, 4, 4, 8, 8};
+static const int kTileCW[6] = {12, 16, 18, 24, 16, 10}, kTileW[6] = {4, 4, 4, 4, 8, 16};
 static int tile_of(int n) {
     int t = 0;
     while (t < 5 && kTileCap[t] < n) ++t;
     return t;
 }
-static size_t lu32_smem(int n, int t) { return (size_t)lu32_layout(n, kTileCW[t], kTileW[t], t != 5).end * 4 + 16; }
+static size_t lu32_smem(int n, int t) { return (size_t)lu32_layout(n, kTileCW[t], kTileW[t]).end * 4 + 16; }
 
 // vk_set_launch's variants: the smallest tiling that covers this many species
 static const int kVariantCap[6] = {48, 80, 112, 160, 128, 128};
@@ -342,8 +341,8 @@ int lu32_tiling_cap(int v) { return v >= 0 && v < 6 ? kVariantCap[v] : 0; }
 cudaError_t init_lu32(int n) {
     cudaError_t e = cudaSuccess;
     int t = 0;
-#define SETATTR(RA, CW, W, DB) \
-    if (e == cudaSuccess && kTileCap[t] >= n) e = raise_smem_limit(k_lu32<RA, CW, W, DB>, lu32_smem(n, t)); \
+#define SETATTR(RA, CW, W) \
+    if (e == cudaSuccess && kTileCap[t] >= n) e = raise_smem_limit(k_lu32<RA, CW, W>, lu32_smem(n, t)); \
     ++t;
     VK_LU32_TILINGS(SETATTR)
 #undef SETATTR
@@ -360,9 +359,9 @@ void launch_lu32(const DevNet &net, const DevBatch &b, const Work &w, cudaStream
     reset_queue(b, s);
     const int grid = half_grid(b, VK_TUNE_LU32, tile < 3 ? 4 : tile == 3 ? 3 : 1);
     int t = 0;
-#define LAUNCH(RA, CW, W, DB)                                                                                  \
+#define LAUNCH(RA, CW, W)                                                                                      \
     if (t++ == tile)                                                                                           \
-        k_lu32<RA, CW, W, DB><<<grid, 32 * W, sm, s>>>(net, b, w.D32, w.dB, w.dC, w.rs, w.cs, w.G32, w.status);
+        k_lu32<RA, CW, W><<<grid, 32 * W, sm, s>>>(net, b, w.D32, w.dB, w.dC, w.rs, w.cs, w.G32, w.status);
     VK_LU32_TILINGS(LAUNCH)
 #undef LAUNCH
 }
