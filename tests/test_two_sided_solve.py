@@ -77,7 +77,7 @@ def test_batch_size_does_not_change_a_column(name):
     atoms = items[0][0].atom_list
     items = [it for _, it in items]
     ref = None
-    for ncols in (3, 15, 33, 90):
+    for ncols in (3, 15, 33, 50, 75, 90):
         sols, delta = _attempt(net, atoms, [items[c % 3] for c in range(ncols)], 1e-7)
         if ref is None:
             ref = (sols, delta)

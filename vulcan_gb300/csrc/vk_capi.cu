@@ -2,6 +2,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <functional>
 #include <cstdio>
 #include <cstring>
 #include <new>
@@ -77,6 +78,7 @@ struct vk_handle {
     cudaStream_t stream2 = nullptr;     // FP64 branch of a mixed attempt (routed columns)
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     int nsm = 0;                        // SMs of the device
+    int nlong = 0;                      // long half-columns of the batch (lu64_long)
     int ncl_lu[3] = {}, ncl_sweep[3] = {};      // clusters it holds at once
     int cps = 0;                        // VK_CTAS_PER_SM override (0: kernel defaults)
     int cps_k[VK_TUNE_N] = {0, 0, 0, 0}; // vk_set_launch: CTAs per SM per kernel
@@ -119,6 +121,7 @@ struct vk_handle {
         b.active = nullptr;
         b.order = d_order;
         b.queue = d_queue;
+        b.nlong = nlong;
         b.nsm = nsm;
         for (int i = 0; i < 3; ++i) {
             b.ncl_lu[i] = ncl_lu[i];
@@ -327,8 +330,8 @@ extern "C" int vk_create(const vk_network *net, int max_cols, int max_layers, in
     TRY(dalloc(h, &h->d_col_end, max_cols));
     TRY(dalloc(h, &h->d_cols, max_cols));
     TRY(dalloc(h, &h->d_order, max_cols));
-    TRY(dalloc(h, &h->d_queue, 1 + max_cols));
-    TRY(dalloc(h, &h->d_queue2, 1 + max_cols));
+    TRY(dalloc(h, &h->d_queue, 2 + max_cols));
+    TRY(dalloc(h, &h->d_queue2, 2 + max_cols));
     TRY(cudaStreamCreateWithFlags(&h->stream2, cudaStreamNonBlocking) == cudaSuccess
             ? VK_OK : fail(h, VK_ECUDA, "cudaStreamCreate (FP64 branch)"));
     TRY(cudaEventCreateWithFlags(&h->ev_fork, cudaEventDisableTiming) == cudaSuccess
@@ -509,7 +512,15 @@ static int set_columns_impl(vk_handle *h, int ncols, int slot_cap, const int *nz
     }
     VK_CUDA(h, cudaMemcpyAsync(h->d_spf, spf, (size_t)ncols * VK_SP_NF * ni * sizeof(double), cudaMemcpyHostToDevice, s));
     VK_CUDA(h, cudaStreamSynchronize(s));
-    if (h->ncols != ncols || h->L != L) drop_graph(h);
+    // (slots are refilled with other lengths)
+    int nlong = 0;
+    if (!slot_cap) {
+        std::vector<int> len(nz, nz + ncols);
+        std::sort(len.begin(), len.end(), std::greater<int>());
+        nlong = vk::lu64_long(h->ni, h->nsm, h->ncl_lu[0], ncols, len.data());
+    }
+    if (h->ncols != ncols || h->L != L || h->nlong != nlong) drop_graph(h);
+    h->nlong = nlong;
     h->ncols = ncols;
     h->L = L;
     h->col_off = off;

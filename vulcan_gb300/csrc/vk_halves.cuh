@@ -22,14 +22,14 @@ __device__ __forceinline__ void cluster_sync_all() {
     asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
 }
 
-// The next unit, -1 when the queue is empty.  All threads call it; in a cluster
-// (CL) every CTA gets rank 0's.
+// The next of `units` from a counter, -1 when there is none left.  All threads
+// call it; in a cluster (CL) every CTA gets rank 0's.
 template <bool CL>
-__device__ __forceinline__ int next_half(const DevBatch &b, int *s_unit, int rank, int csize) {
+__device__ __forceinline__ int next_unit(unsigned *queue, int units, int *s_unit, int rank, int csize) {
     if (CL) {
         cluster_sync_all();
         if (rank == 0 && threadIdx.x == 0) {
-            const int u = (int)atomicAdd(b.queue, 1u);
+            const int u = (int)atomicAdd(queue, 1u);
             const uint32_t la = smem_u32(s_unit);
             for (int d = 0; d < csize; ++d)
                 asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(cluster_addr(la, (uint32_t)d)), "r"(u) : "memory");
@@ -37,11 +37,15 @@ __device__ __forceinline__ int next_half(const DevBatch &b, int *s_unit, int ran
         cluster_sync_all();
     } else {
         __syncthreads();
-        if (threadIdx.x == 0) *s_unit = (int)atomicAdd(b.queue, 1u);
+        if (threadIdx.x == 0) *s_unit = (int)atomicAdd(queue, 1u);
         __syncthreads();
     }
     const int u = *s_unit;
-    return u < 2 * b.ncols ? u : -1;
+    return u < units ? u : -1;
+}
+template <bool CL>
+__device__ __forceinline__ int next_half(const DevBatch &b, int *s_unit, int rank, int csize) {
+    return next_unit<CL>(b.queue, 2 * b.ncols, s_unit, rank, csize);
 }
 
 // True for the second of a column's halves to get here; what the first wrote
@@ -78,9 +82,9 @@ inline int half_grid(const DevBatch &b, int kernel, int cps_default) {
     return (g > 0 && g < 2ll * b.ncols) ? (int)g : 2 * b.ncols;
 }
 
-// Zero the queue position and the columns' arrival counts.
+// Zero the queue position, the columns' arrival counts and the second position.
 inline void reset_queue(const DevBatch &b, cudaStream_t s) {
-    cudaMemsetAsync(b.queue, 0, (size_t)(1 + b.ncols) * sizeof(unsigned), s);
+    cudaMemsetAsync(b.queue, 0, (size_t)(2 + b.ncols) * sizeof(unsigned), s);
 }
 
 }  // namespace vk

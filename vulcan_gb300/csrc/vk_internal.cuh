@@ -119,8 +119,10 @@ struct DevBatch {
     const double *spf;         // [ncols][VK_SP_NF][ni]
     const int *active;         // [ncols] non-zero = column takes part (NULL = all)
     const int *order;          // [ncols] columns by decreasing nz (work-queue order)
-    unsigned *queue;           // [1 + ncols] next queue position, then per column how many of
-                               //  its halves are done (zeroed before each launch)
+    unsigned *queue;           // [2 + ncols] next queue position, per column how many of its
+                               //  halves are done, a second position (zeroed before each launch)
+    int nlong;                 // half-columns the FP64 factorisation shares between two CTAs
+                               //  when it gives the others one each (lu64_long)
     int nsm;                   // SMs of the device
     int ncl_lu[3], ncl_sweep[3];    // clusters of 2, 4, 8 CTAs it holds at once (vk_lu64.cu)
     int cps;                   // resident CTAs per SM of the per-column kernels
@@ -245,6 +247,7 @@ void launch_rates(const DevNet &net, const DevBatch &b, const double *y, double 
 void launch_geometry(const DevNet &net, const DevBatch &b, double *geo, int flags, cudaStream_t s);
 cudaError_t init_lu64(int n);
 void cluster_limits(int n, int lu[3], int sweep[3]);
+int lu64_long(int n, int nsm, int clusters2, int ncols, const int *nz);
 void launch_lu64(const DevNet &net, const DevBatch &b, const Work &w, cudaStream_t s);
 // One column of given blocks (sizes and words: vk_lu64.cu).
 constexpr int kSolve64Words = 8;

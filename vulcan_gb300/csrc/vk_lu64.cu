@@ -19,13 +19,16 @@
 // of dependent pivots (vk_lu64.cuh) when they do not: then the CTAs of a
 // cluster share each block.  Measured against the one-sided factorisation,
 // one CTA per column, that it replaced (ms, GB300): one CHO column of 100
-// layers 6.1 -> 1.5, one NCHO column of 150 layers 21.4 -> 4.2, 64 uneven NCHO
-// columns 28.0 -> 12.2, 512 50.6 -> 46.0.  The sweeps are bound by the FP64
+// layers 6.1 -> 1.4, one NCHO column of 150 layers 21.4 -> 3.7, 64 uneven NCHO
+// columns 28.0 -> 10.2, 512 50.6 -> 46.0.  The sweeps are bound by the FP64
 // products of a layer and the latency between dependent layers.
 //
 // Reference: the banded LU of the Ros2 LHS, op.py:2913-2929.
 #include <cuda_runtime.h>
 #include <math.h>
+
+#include <algorithm>
+#include <functional>
 
 #include "vk_internal.cuh"
 #include "vk_halves.cuh"
@@ -37,6 +40,7 @@ namespace vk {
 namespace {
 
 constexpr size_t kMaxSmem = 232448;    // dynamic shared memory of a CTA
+constexpr int kLongMax = 256;          // most half-columns lu64_long looks at
 
 __host__ __device__ inline size_t lu64_smem(int n, int csize) {
     const int w = lu64_slice_max(n, csize);
@@ -46,9 +50,157 @@ __host__ __device__ inline size_t lu64_smem(int n, int csize) {
 
 }  // namespace
 
+namespace {
+
+// This CTA's part of the shared memory at sm and of the blocks (rank of csize).
+template <bool CL>
+__device__ __forceinline__ Lu64Mem lu64_mem(double *sm, int n, int csize, int rank, int *s_sing, int *s_dead) {
+    Lu64Mem m;
+    m.n = n;
+    m.csize = CL ? csize : 1;
+    m.rank = CL ? rank : 0;
+    m.pw = lu64_prep_warps(n);
+    m.c0 = lu64_slice(n, m.csize, m.rank);
+    m.w = lu64_slice(n, m.csize, m.rank + 1) - m.c0;
+    m.S = sm;
+    m.msg = m.S + ((n * lu64_slice_max(n, m.csize) + 1) & ~1);
+    m.srow = m.msg + (CL ? n : 2) * lu64_msg(n);
+    m.rowf = m.srow + n;
+    m.colf = m.rowf + n;
+    m.diag = m.colf + n;
+    m.xval = m.diag + n;
+    m.xkey = reinterpret_cast<unsigned *>(m.xval + 8);
+    m.bar = reinterpret_cast<uint64_t *>(m.xkey + 8);
+    m.rowid = reinterpret_cast<int *>(m.bar + n);
+    m.colid = m.rowid + n;
+    m.perm = m.colid + n;
+    m.kinv = m.perm + n;
+    m.sing = s_sing;
+    m.dead = s_dead;
+    return m;
+}
+
+// The half-column u (and the column's middle, if it is the second half).
 // DENSE: the blocks are given, jv = D [layer][n][n], and so are the couplings
 // (their sign cancels in the Schur terms); the inverses are packed (stride n n).
-// mid1: the middle layer, nz / 2 if negative.
+// mid1: the middle layer, nz / 2 if negative.  phase: inversions so far.
+template <bool CL, bool DENSE>
+__device__ __forceinline__ void lu64_half(const DevNet &net, const DevBatch &b, const Lu64Mem &m,
+                                          const double *__restrict__ jv, const double *__restrict__ dA,
+                                          const double *__restrict__ dB, const double *__restrict__ dC,
+                                          const double *__restrict__ dt, double *G, int *status, int mid1, int u,
+                                          int *s_unit, unsigned &phase) {
+    const int n = net.ni, gst = DENSE ? n * n : block_stride64(n);
+    const int tid = threadIdx.x, nth = blockDim.x;
+    const int w = m.w, c0s = m.c0, ne = n * w;
+    int *rowpos = m.perm, *colpos = m.kinv;            // free between inversions
+    const int c = b.order[u >> 1], half = u & 1;
+    if (b.active && !b.active[c]) return;
+    const int l0 = b.col_off[c], nz = b.col_end[c] - l0, mid = mid1 >= 0 ? mid1 : nz / 2;
+    const int cnt = half ? nz - 1 - mid : mid;
+    const double cdt = DENSE ? 0.0 : 1.0 / (R_ROS * dt[c]);
+    if (tid == 0) *m.sing = 0;
+    for (int t = tid; t < n; t += nth) { m.rowid[t] = t; m.colid[t] = t; }
+    __syncthreads();
+    bool middle = false;
+    // t < cnt: the half's layers; t == cnt: the last inverse is stored and,
+    // for the second half to get there, the middle layer follows
+    for (int t = 0; t <= cnt || middle; ++t) {
+        const int j = middle ? mid : (half ? nz - 1 - t : t);
+        const size_t l = (size_t)l0 + j;
+        const bool build = t < cnt || middle;
+        const double *Dl = DENSE ? jv + l * gst : nullptr;
+        if (build) {
+            const double *rf = half ? dB + l * n : dC + l * n;
+            const double *cf = half ? dC + (l + 1) * n : dB + (l - 1) * n;
+            for (int q = tid; q < n; q += nth) {
+                if (!DENSE) m.diag[q] = cdt - dA[l * n + q];
+                if (t > 0 && !middle) {
+                    m.rowf[q] = -rf[m.rowid[q]] * m.srow[q];
+                    m.colf[q] = cf[m.colid[q]];
+                }
+            }
+        }
+        __syncthreads();
+        if (middle) {
+            // natural order; both neighbours' inverses from global memory
+            const double *Gd = G + (l - 1) * gst, *Gu = G + (l + 1) * gst;
+            const bool down = mid > 0, up = mid + 1 < nz;
+            for (int e = tid; e < ne; e += nth) {
+                const int r = e / w, q = c0s + e - r * w;
+                double v = down ? -dC[l * n + r] * __ldcg(Gd + r * n + q) * dB[(l - 1) * n + q] : 0.0;
+                if (up) v -= dB[l * n + r] * __ldcg(Gu + r * n + q) * dC[(l + 1) * n + q];
+                if (DENSE) v += Dl[r * n + q];
+                else if (r == q) v += m.diag[r];
+                m.S[e] = v;
+            }
+        } else if (t == 0) {
+            if (build) for (int e = tid; e < ne; e += nth) {
+                const int r = e / w, q = c0s + e - r * w;
+                m.S[e] = DENSE ? Dl[r * n + q] : r == q ? m.diag[r] : 0.0;
+            }
+        } else {
+            // store the previous layer's inverse and replace it by this layer's Schur term
+            double *Gp = G + (l + (half ? 1 : -1)) * (long long)gst;
+            for (int e = tid; e < ne; e += nth) {
+                const int r = e / w, q = c0s + e - r * w;
+                const int ri = m.rowid[r], ci = m.colid[q];
+                const double s = m.S[e];
+                Gp[ri * n + ci] = s * m.srow[r];
+                if (build) {
+                    double v = s * m.rowf[r] * m.colf[q];
+                    if (DENSE) v += Dl[ri * n + ci];
+                    else if (ri == ci) v += m.diag[ri];
+                    m.S[e] = v;
+                }
+            }
+        }
+        if (build) {
+            if (!DENSE) {
+                for (int q = tid; q < n; q += nth) {
+                    rowpos[m.rowid[q]] = q;
+                    colpos[m.colid[q]] = q - c0s;
+                }
+                __syncthreads();
+                const double *jl = jv + l * net.nnz;
+                for (int e = tid; e < net.nnz; e += nth) {
+                    const int q = colpos[net.jcol[e]];
+                    if (!CL || (unsigned)q < (unsigned)w) m.S[rowpos[net.jrow[e]] * w + q] += jl[e];
+                }
+            }
+            __syncthreads();
+            lu64_invert<CL>(m, phase);
+            ++phase;
+        }
+        if (middle) {
+            double *Gl = G + l * gst;
+            for (int e = tid; e < ne; e += nth) {
+                const int r = e / w, q = c0s + e - r * w;
+                Gl[m.rowid[r] * n + m.colid[q]] = m.S[e] * m.srow[r];
+            }
+            break;
+        }
+        if (t == cnt) {
+            middle = second_half<CL>(b, c, s_unit, m.rank, m.csize);
+            if (!middle) break;
+            for (int q = tid; q < n; q += nth) { m.rowid[q] = q; m.colid[q] = q; }
+            __syncthreads();
+        }
+    }
+    if (tid == 0 && *m.dead) atomicExch(&status[c], VK_ETIMEOUT);
+    else if (tid == 0 && m.rank == 0 && *m.sing)
+        atomicCAS(&status[c], 0, *m.sing == 2 ? VK_ENAN : VK_ESINGULAR);
+}
+
+// The message barriers of a cluster.
+__device__ __forceinline__ void lu64_open(const Lu64Mem &m) {
+    for (int k = threadIdx.x; k < m.n; k += blockDim.x) mbar_init(&m.bar[k], 1);
+    mbar_fence_init();
+    cluster_sync_all();
+}
+
+}  // namespace
+
 template <bool CL, bool DENSE>
 __global__ void __launch_bounds__(CL ? 384 : 544, CL ? 1 : 2)
 k_lu64(DevNet net, DevBatch b, const double *__restrict__ jv, const double *__restrict__ dA,
@@ -56,138 +208,35 @@ k_lu64(DevNet net, DevBatch b, const double *__restrict__ jv, const double *__re
        const double *__restrict__ dt, double *G, int *status, int csize, int mid1) {
     extern __shared__ __align__(16) double sm[];
     __shared__ int s_unit, s_sing, s_dead;
-    const int n = net.ni, gst = DENSE ? n * n : block_stride64(n);
-    const int tid = threadIdx.x, nth = blockDim.x;
-    Lu64Mem m;
-    m.n = n;
-    m.csize = CL ? csize : 1;
-    m.rank = CL ? (int)cluster_rank() : 0;
-    m.pw = lu64_prep_warps(n);
-    m.c0 = lu64_slice(n, m.csize, m.rank);
-    m.w = lu64_slice(n, m.csize, m.rank + 1) - m.c0;
-    m.S = sm;
-    m.msg = m.S + ((n * lu64_slice_max(n, m.csize) + 1) & ~1);
-    m.srow = m.msg + (CL ? n : 2) * lu64_msg(n);
-    double *rowf = m.srow + n;             // [n] row factors of the Schur term, by stored row
-    double *colf = rowf + n;               // [n] column factors, by stored column
-    double *diag = colf + n;               // [n] c0 - dA, by species
-    m.xval = diag + n;
-    m.xkey = reinterpret_cast<unsigned *>(m.xval + 8);
-    m.bar = reinterpret_cast<uint64_t *>(m.xkey + 8);
-    m.rowid = reinterpret_cast<int *>(m.bar + n);
-    m.colid = m.rowid + n;
-    m.perm = m.colid + n;
-    m.kinv = m.perm + n;
-    m.sing = &s_sing;
-    m.dead = &s_dead;
-    const int w = m.w, c0s = m.c0, ne = n * w;
-    int *rowpos = m.perm, *colpos = m.kinv;            // free between inversions
-    if (tid == 0) s_dead = 0;
-    if (CL) {
-        for (int k = tid; k < n; k += nth) mbar_init(&m.bar[k], 1);
-        mbar_fence_init();
+    const Lu64Mem m = lu64_mem<CL>(sm, net.ni, csize, CL ? (int)cluster_rank() : 0, &s_sing, &s_dead);
+    if (threadIdx.x == 0) s_dead = 0;
+    if (CL) lu64_open(m);
+    unsigned phase = 0;
+    for (int u; (u = next_half<CL>(b, &s_unit, m.rank, m.csize)) >= 0;)
+        lu64_half<CL, DENSE>(net, b, m, jv, dA, dB, dC, dt, G, status, mid1, u, &s_unit, phase);
+    if (CL) cluster_sync_all();            // no message is still on its way to a CTA that has left
+}
+
+// Clusters of two: the longest nlong half-columns are each shared by a
+// cluster, then every CTA goes on alone (lu64_long).
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(544, 1)
+k_lu64_long(DevNet net, DevBatch b, const double *__restrict__ jv, const double *__restrict__ dA,
+            const double *__restrict__ dB, const double *__restrict__ dC,
+            const double *__restrict__ dt, double *G, int *status) {
+    extern __shared__ __align__(16) double sm[];
+    __shared__ int s_unit, s_sing, s_dead;
+    unsigned phase = 0;
+    if (threadIdx.x == 0) s_dead = 0;
+    {
+        const Lu64Mem m = lu64_mem<true>(sm, net.ni, 2, (int)cluster_rank(), &s_sing, &s_dead);
+        lu64_open(m);
+        for (int u; (u = next_unit<true>(b.queue, b.nlong, &s_unit, m.rank, 2)) >= 0;)
+            lu64_half<true, false>(net, b, m, jv, dA, dB, dC, dt, G, status, -1, u, &s_unit, phase);
         cluster_sync_all();
     }
-    unsigned phase = 0;
-    for (int u; (u = next_half<CL>(b, &s_unit, m.rank, m.csize)) >= 0;) {
-        const int c = b.order[u >> 1], half = u & 1;
-        if (b.active && !b.active[c]) continue;
-        const int l0 = b.col_off[c], nz = b.col_end[c] - l0, mid = mid1 >= 0 ? mid1 : nz / 2;
-        const int cnt = half ? nz - 1 - mid : mid;
-        const double cdt = DENSE ? 0.0 : 1.0 / (R_ROS * dt[c]);
-        if (tid == 0) s_sing = 0;
-        for (int t = tid; t < n; t += nth) { m.rowid[t] = t; m.colid[t] = t; }
-        __syncthreads();
-        bool middle = false;
-        // t < cnt: the half's layers; t == cnt: the last inverse is stored and,
-        // for the second half to get there, the middle layer follows
-        for (int t = 0; t <= cnt || middle; ++t) {
-            const int j = middle ? mid : (half ? nz - 1 - t : t);
-            const size_t l = (size_t)l0 + j;
-            const bool build = t < cnt || middle;
-            const double *Dl = DENSE ? jv + l * gst : nullptr;
-            if (build) {
-                const double *rf = half ? dB + l * n : dC + l * n;
-                const double *cf = half ? dC + (l + 1) * n : dB + (l - 1) * n;
-                for (int q = tid; q < n; q += nth) {
-                    if (!DENSE) diag[q] = cdt - dA[l * n + q];
-                    if (t > 0 && !middle) {
-                        rowf[q] = -rf[m.rowid[q]] * m.srow[q];
-                        colf[q] = cf[m.colid[q]];
-                    }
-                }
-            }
-            __syncthreads();
-            if (middle) {
-                // natural order; both neighbours' inverses from global memory
-                const double *Gd = G + (l - 1) * gst, *Gu = G + (l + 1) * gst;
-                const bool down = mid > 0, up = mid + 1 < nz;
-                for (int e = tid; e < ne; e += nth) {
-                    const int r = e / w, q = c0s + e - r * w;
-                    double v = down ? -dC[l * n + r] * __ldcg(Gd + r * n + q) * dB[(l - 1) * n + q] : 0.0;
-                    if (up) v -= dB[l * n + r] * __ldcg(Gu + r * n + q) * dC[(l + 1) * n + q];
-                    if (DENSE) v += Dl[r * n + q];
-                    else if (r == q) v += diag[r];
-                    m.S[e] = v;
-                }
-            } else if (t == 0) {
-                if (build) for (int e = tid; e < ne; e += nth) {
-                    const int r = e / w, q = c0s + e - r * w;
-                    m.S[e] = DENSE ? Dl[r * n + q] : r == q ? diag[r] : 0.0;
-                }
-            } else {
-                // store the previous layer's inverse and replace it by this layer's Schur term
-                double *Gp = G + (l + (half ? 1 : -1)) * (long long)gst;
-                for (int e = tid; e < ne; e += nth) {
-                    const int r = e / w, q = c0s + e - r * w;
-                    const int ri = m.rowid[r], ci = m.colid[q];
-                    const double s = m.S[e];
-                    Gp[ri * n + ci] = s * m.srow[r];
-                    if (build) {
-                        double v = s * rowf[r] * colf[q];
-                        if (DENSE) v += Dl[ri * n + ci];
-                        else if (ri == ci) v += diag[ri];
-                        m.S[e] = v;
-                    }
-                }
-            }
-            if (build) {
-                if (!DENSE) {
-                    for (int q = tid; q < n; q += nth) {
-                        rowpos[m.rowid[q]] = q;
-                        colpos[m.colid[q]] = q - c0s;
-                    }
-                    __syncthreads();
-                    const double *jl = jv + l * net.nnz;
-                    for (int e = tid; e < net.nnz; e += nth) {
-                        const int q = colpos[net.jcol[e]];
-                        if (!CL || (unsigned)q < (unsigned)w) m.S[rowpos[net.jrow[e]] * w + q] += jl[e];
-                    }
-                }
-                __syncthreads();
-                lu64_invert<CL>(m, phase);
-                ++phase;
-            }
-            if (middle) {
-                double *Gl = G + l * gst;
-                for (int e = tid; e < ne; e += nth) {
-                    const int r = e / w, q = c0s + e - r * w;
-                    Gl[m.rowid[r] * n + m.colid[q]] = m.S[e] * m.srow[r];
-                }
-                break;
-            }
-            if (t == cnt) {
-                middle = second_half<CL>(b, c, &s_unit, m.rank, m.csize);
-                if (!middle) break;
-                for (int q = tid; q < n; q += nth) { m.rowid[q] = q; m.colid[q] = q; }
-                __syncthreads();
-            }
-        }
-        if (tid == 0 && s_dead) atomicExch(&status[c], VK_ETIMEOUT);
-        else if (tid == 0 && m.rank == 0 && s_sing)
-            atomicCAS(&status[c], 0, s_sing == 2 ? VK_ENAN : VK_ESINGULAR);
-    }
-    if (CL) cluster_sync_all();            // no message is still on its way to a CTA that has left
+    const Lu64Mem m = lu64_mem<false>(sm, net.ni, 1, 0, &s_sing, &s_dead);
+    for (int u; (u = next_unit<false>(b.queue + 1 + b.ncols, 2 * b.ncols - b.nlong, &s_unit, 0, 1)) >= 0;)
+        lu64_half<false, false>(net, b, m, jv, dA, dB, dC, dt, G, status, -1, b.nlong + u, &s_unit, phase);
 }
 
 // One FP64 sweep over half-columns.  FWD: towards the middle,
@@ -561,7 +610,7 @@ struct ClusterLaunch {
 
 // CTAs per half-column.  While the half-columns do not fill the chip, sharing
 // each block between the CTAs of a cluster shortens the chain of its pivots
-// (one NCHO column: 9.8, 6.5, 5.0 and 4.2 ms with 1, 2, 4 and 8); the line
+// (one NCHO column: 9.5, 6.7, 4.7 and 3.7 ms with 1, 2, 4 and 8); the line
 // lies where every CTA still has an SM of its own, because beyond it the
 // shared FP64 units gain nothing (64 columns: 12.2, 12.4, 18.1 and 36.5 ms),
 // and where the device holds all the clusters at once: an SM count that a
@@ -605,6 +654,7 @@ cudaError_t init_lu64(int n) {
     }
     cudaError_t e = raise_smem_limit(k_lu64<false, false>, lu64_smem(n, 1));
     if (e == cudaSuccess && scl) e = raise_smem_limit(k_lu64<true, false>, scl);
+    if (e == cudaSuccess && lu64_fits(n, 2)) e = raise_smem_limit(k_lu64_long, std::max(lu64_smem(n, 1), lu64_smem(n, 2)));
     const size_t ssw = sweep64_smem(n, sweep64_nbuf(n, 1));
     if (e == cudaSuccess) e = raise_smem_limit(k_sweep64<true>, ssw);
     if (e == cudaSuccess) e = raise_smem_limit(k_sweep64<false>, ssw);
@@ -613,9 +663,48 @@ cudaError_t init_lu64(int n) {
     return e;
 }
 
+// How many of the half-columns (lengths by decreasing nz, two to a column) a
+// cluster should share while every CTA has an SM of its own but not a cluster: the
+// number that makes the last CTA finish first, by the steps' costs in cycles (the
+// FP64 unit's 19 per warp-wide instruction, and what a step waits for).  NCHO
+// columns of 60 to 200 layers, without and with it: 40 columns 12.3 and 8.4 ms, 64
+// columns 12.2 and 10.2, 76 columns 12.7 and 10.8.
+int lu64_long(int n, int nsm, int clusters2, int ncols, const int *nz) {
+    const int units = 2 * ncols, ncl = std::min(clusters2, nsm / 2), lim = kLongMax;
+    if (!lu64_fits(n, 2) || units > 2 * ncl || 2 * units <= nsm || units > lim) return 0;
+    const int pw = lu64_prep_warps(n);
+    const double one = 19. * (n * n / 32. + 3 * pw) + 560, two = 19. * (n * n / 64. + 5 * pw) + 900;
+    int best = 0;
+    double tbest = 0;
+    double cl[kLongMax], cta[2 * kLongMax];
+    // to whoever is free first (v a heap, the earliest on top)
+    auto assign = [](double *v, int k, double cost) {
+        std::pop_heap(v, v + k, std::greater<double>());
+        v[k - 1] += cost;
+        std::push_heap(v, v + k, std::greater<double>());
+    };
+    for (int a = 0; a <= units; a += 4) {
+        std::fill(cl, cl + ncl, 0.);
+        for (int u = 0; u < a; ++u) assign(cl, ncl, two * (nz[u / 2] / 2));
+        for (int i = 0; i < 2 * ncl; ++i) cta[i] = cl[i / 2];
+        std::make_heap(cta, cta + 2 * ncl, std::greater<double>());
+        for (int u = a; u < units; ++u) assign(cta, 2 * ncl, one * (nz[u / 2] / 2));
+        const double t = *std::max_element(cta, cta + 2 * ncl);
+        if (a == 0 || t < 0.97 * tbest) { tbest = t; best = a; }
+    }
+    return best;
+}
+
 void launch_lu64(const DevNet &net, const DevBatch &b, const Work &w, cudaStream_t s) {
     const int n = net.ni, cs = cluster_size(b, b.ncl_lu, lu64_fits, n);
     reset_queue(b, s);
+    if (b.nlong > 0 && cs == 1 && b.cps == 0 && b.cps_k[VK_TUNE_LU64] == 0) {
+        const ClusterLaunch L(std::min(b.ncl_lu[0], b.nsm / 2) * 2, lu64_threads(n, 1),
+                              std::max(lu64_smem(n, 1), lu64_smem(n, 2)), 1, s);
+        cudaLaunchKernelEx(&L.cfg, k_lu64_long, net, b, (const double *)w.jv, (const double *)w.dA,
+                           (const double *)w.dB, (const double *)w.dC, (const double *)w.dt, w.G, w.status);
+        return;
+    }
     const ClusterLaunch L(cs == 1 ? half_grid(b, VK_TUNE_LU64, 2) : 2 * b.ncols * cs, lu64_threads(n, cs),
                           lu64_smem(n, cs), cs, s);
     cudaLaunchKernelEx(&L.cfg, cs == 1 ? k_lu64<false, false> : k_lu64<true, false>, net, b, (const double *)w.jv,

@@ -98,6 +98,8 @@ struct Lu64Mem {
     double *S;            // [n][w] this CTA's columns
     double *msg;          // [nslot][lu64_msg] 1/pivot, pivot row + flag, multipliers
     double *srow;         // [n] scale of each stored row
+    double *rowf, *colf;  // [n] factors of the Schur term, by stored row and column
+    double *diag;         // [n] c0 - dA, by species
     double *xval;         // [8] the prep warps' candidates' reciprocals
     unsigned *xkey;       // [8] and keys (16-byte aligned; zero beyond the prep warps)
     int *rowid, *colid;   // [n] labels

@@ -14,7 +14,7 @@
 //     lower[j] o x[j-1] + D[j] x[j] + upper[j] o x[j+1] = b[j]
 // (D dense ni x ni, lower/upper diagonal vectors) with the FP64 solver's
 // two-sided block-Thomas (vk_lu64.cu): a cluster of eight CTAs per half of the
-// column.  A column of 150 layers of 69 species: 28.1 -> 4.4 ms (one CTA from
+// column.  A column of 150 layers of 69 species: 28.1 -> 3.7 ms (one CTA from
 // one end before).  Where the two-sided order meets a block without a finite
 // non-zero pivot, the column is solved once more from its bottom alone, whose
 // answer or failure is the call's.
