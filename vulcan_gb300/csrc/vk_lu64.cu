@@ -610,7 +610,7 @@ struct ClusterLaunch {
 
 // CTAs per half-column.  While the half-columns do not fill the chip, sharing
 // each block between the CTAs of a cluster shortens the chain of its pivots
-// (one NCHO column: 9.5, 6.7, 4.7 and 3.7 ms with 1, 2, 4 and 8); the line
+// (one NCHO column: 9.5, 6.7, 4.5 and 3.7 ms with 1, 2, 4 and 8); the line
 // lies where every CTA still has an SM of its own, because beyond it the
 // shared FP64 units gain nothing (64 columns: 12.2, 12.4, 18.1 and 36.5 ms),
 // and where the device holds all the clusters at once: an SM count that a

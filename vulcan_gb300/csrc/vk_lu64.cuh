@@ -44,8 +44,8 @@ constexpr int kLu64MinCluster = 32;    // smallest block a cluster may share
 __host__ __device__ inline int lu64_prep_warps(int n) { return (n + 31) / 32; }
 // Bulk warps of a CTA that has a block to itself, as many on each of the SM's
 // four schedulers (512 NCHO columns: 6, 8, 10, 12 and 14 warps 49.4, 49.5, 47.1,
-// 46.0 and 47.4 ms), and of a cluster's (one column: 6, 7, 12 warps 4.41, 4.21
-// and 4.17 ms, seven of 89 species 8.46, 8.16 and 8.49).
+// 46.0 and 47.4 ms), and of a cluster's (5 to 9 warps: one NCHO column 4.09, 4.03,
+// 3.72, 3.82 and 3.82 ms, seven columns of 89 species 5.46, 5.24, 5.09, 5.28 and 5.24).
 __host__ __device__ inline int lu64_threads(int n, int csize) {
     return 32 * (lu64_prep_warps(n) + (csize > 1 ? 7 : 12));
 }
