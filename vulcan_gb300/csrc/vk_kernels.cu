@@ -259,25 +259,40 @@ k_stage(DevNet net, DevBatch b, const double *__restrict__ y, const double *__re
     }
 }
 
-// Transport geometry of every (layer, species) of the active columns.
+// Transport geometry of every (layer, species) of the active columns, a CTA per
+// kGeoTile layers.  FP64 divisions bound it: those of a layer alone are done
+// once a layer, 10 of 28 are left per species.  66 752 layers of 69 species
+// 1.88 -> 1.08 ms (every division per species before).
+constexpr int kGeoTile = 8;
 __global__ void __launch_bounds__(256)
 k_geometry(DevNet net, DevBatch b, double *__restrict__ geo, int flags) {
-    const int ni = net.ni;
-    const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= (long long)b.L * ni) return;
-    const int l = (int)(e / ni), i = (int)(e - (long long)l * ni);
-    const int c = b.lay_col[l];
-    if (c < 0 || (b.active && !b.active[c])) return;
-    const GeoCol cv = make_geocol(b.atm, b.Dzz, b.spf, b.col_off, b.col_end, c, ni);
-    double out[GEO_NF];
-    geo_coef(cv, l - cv.l0, i, flags, out);
-    double *gl = geo + (size_t)l * GEO_NF * ni;
-    for (int k = 0; k < GEO_NF; ++k) gl[k * ni + i] = out[k];
+    __shared__ GeoLayer lay[kGeoTile];
+    const int ni = net.ni, lt = blockIdx.x * kGeoTile;
+    auto column = [&](int l) {             // -1: no work
+        const int c = l < b.L ? b.lay_col[l] : -1;
+        return c >= 0 && !(b.active && !b.active[c]) ? c : -1;
+    };
+    if (threadIdx.x < kGeoTile) {
+        const int l = lt + threadIdx.x, c = column(l);
+        if (c >= 0) {
+            const GeoCol cv = make_geocol(b.atm, b.Dzz, b.spf, b.col_off, b.col_end, c, ni);
+            lay[threadIdx.x] = geo_layer(cv, l - cv.l0, flags);
+        }
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < kGeoTile * ni; e += blockDim.x) {
+        const int t = e / ni, i = e - t * ni, l = lt + t, c = column(l);
+        if (c < 0) continue;
+        const GeoCol cv = make_geocol(b.atm, b.Dzz, b.spf, b.col_off, b.col_end, c, ni);
+        double out[GEO_NF];
+        geo_species(cv, lay[t], l - cv.l0, i, flags, out);
+        double *gl = geo + (size_t)l * GEO_NF * ni;
+        for (int k = 0; k < GEO_NF; ++k) gl[k * ni + i] = out[k];
+    }
 }
 
 void launch_geometry(const DevNet &net, const DevBatch &b, double *geo, int flags, cudaStream_t s) {
-    long long n = (long long)b.L * net.ni;
-    k_geometry<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(net, b, geo, flags);
+    k_geometry<<<(b.L + kGeoTile - 1) / kGeoTile, 256, 0, s>>>(net, b, geo, flags);
 }
 
 // ---------------------------------------------------------------------------
