@@ -233,6 +233,10 @@ k_lu64_long(DevNet net, DevBatch b, const double *__restrict__ jv, const double 
         for (int u; (u = next_unit<true>(b.queue, b.nlong, &s_unit, m.rank, 2)) >= 0;)
             lu64_half<true, false>(net, b, m, jv, dA, dB, dC, dt, G, status, -1, u, &s_unit, phase);
         cluster_sync_all();
+        // the barriers' memory holds data from here on
+        for (int k = threadIdx.x; k < m.n; k += blockDim.x)
+            asm volatile("mbarrier.inval.shared::cta.b64 [%0];" ::"r"(smem_u32(&m.bar[k])) : "memory");
+        __syncthreads();
     }
     const Lu64Mem m = lu64_mem<false>(sm, net.ni, 1, 0, &s_sing, &s_dead);
     for (int u; (u = next_unit<false>(b.queue + 1 + b.ncols, 2 * b.ncols - b.nlong, &s_unit, 0, 1)) >= 0;)
