@@ -308,6 +308,11 @@ VK_API int  vk_compute_k(vk_handle *h);
 #define VK_TUNE_N       4
 VK_API int  vk_set_launch(vk_handle *h, int kernel, int ctas_per_sm, int variant);
 VK_API int  vk_get_launch(vk_handle *h, int kernel, int *ctas_per_sm, int *variant);
+/* Polls after which a CTA of the FP64 solve stops waiting for another CTA's
+ * message (0..2^22, the built-in limit; < 0 restores it); the column then ends
+ * with VK_ETIMEOUT and nothing of the block is stored.  For tests: with 0 the
+ * first wait gives up. */
+VK_API int  vk_set_wait_limit(vk_handle *h, int polls);
 /* Diagnostic: the device rate constants [L][nr] back to the host. */
 VK_API int  vk_get_k(vk_handle *h, double *k);
 

@@ -42,7 +42,7 @@ EXPORTS = ('vk_network_compile', 'vk_network_info', 'vk_network_jac_pattern', 'v
            'vk_photo_update', 'vk_photo_get', 'vk_photo_set_cross_T', 'vk_set_rate_caps',
            'vk_set_launch', 'vk_get_launch', 'vk_set_conv_ignore', 'vk_get_lu32', 'vk_rhs',
            'vk_set_columns_slotted', 'vk_refill', 'vk_group_create', 'vk_group_run',
-           'vk_group_timing', 'vk_group_destroy')
+           'vk_group_timing', 'vk_group_destroy', 'vk_set_wait_limit')
 
 
 class VkNetworkDesc(C.Structure):
@@ -125,6 +125,7 @@ def lib(path=None):
         'vk_set_rate_caps': (i, [vp, pi, pd, pd]),
         'vk_set_launch': (i, [vp, i, i, i]),
         'vk_get_launch': (i, [vp, i, pi, pi]),
+        'vk_set_wait_limit': (i, [vp, i]),
         'vk_get_k': (i, [vp, pd]),
         'vk_photo_setup': (i, [vp, i, pd, pd, i, pi, pi, pd, i, pi, pd, i, pi, pd, pd,
                                C.c_double, C.c_double, C.c_double, C.c_double]),

@@ -15,6 +15,7 @@
 
 #include "vk_control.cuh"
 #include "vk_internal.cuh"
+#include "vk_tma.cuh"
 
 namespace vk {
 void launch_chem_only(const DevNet &net, const DevBatch &b, const double *y, double *f,
@@ -81,6 +82,7 @@ struct vk_handle {
     int nlong = 0;                      // long half-columns of the batch (lu64_long)
     int ncl_lu[3] = {}, ncl_sweep[3] = {};      // clusters it holds at once
     int cps = 0;                        // VK_CTAS_PER_SM override (0: kernel defaults)
+    int spin = vk::kMbarSpin;           // vk_set_wait_limit
     int cps_k[VK_TUNE_N] = {0, 0, 0, 0}; // vk_set_launch: CTAs per SM per kernel
     int lu32_tiling = -1;               // vk_set_launch: k_lu32 variant (-1: by ni)
     int occ_rates[3] = {}, occ_prep = 0;    // resident CTAs per SM of k_rates (tiles of 1, 2, 4 layers) / k_prep32
@@ -128,6 +130,7 @@ struct vk_handle {
             b.ncl_sweep[i] = ncl_sweep[i];
         }
         b.cps = cps;
+        b.spin = spin;
         for (int i = 0; i < VK_TUNE_N; ++i) b.cps_k[i] = cps_k[i];
         b.lu32_tiling = lu32_tiling;
         for (int i = 0; i < 3; ++i) b.grid_rates[i] = nsm * occ_rates[i];
@@ -992,6 +995,15 @@ extern "C" int vk_set_rate_params(vk_handle *h, const int *kind, const int *rev,
     VK_CUDA(h, cudaMemcpy(h->d_krev, rev, h->npair * sizeof(int), cudaMemcpyHostToDevice));
     VK_CUDA(h, cudaMemcpy(h->d_kpar, params, (size_t)h->npair * 6 * sizeof(double), cudaMemcpyHostToDevice));
     VK_CUDA(h, cudaMemcpy(h->d_nasa9, nasa9, (size_t)h->ni * 20 * sizeof(double), cudaMemcpyHostToDevice));
+    return VK_OK;
+}
+
+extern "C" int vk_set_wait_limit(vk_handle *h, int polls) {
+    if (!h) return fail(nullptr, VK_EINVAL, "handle is NULL");
+    if (polls > vk::kMbarSpin) return fail(h, VK_EINVAL, "polls must be at most " + std::to_string(vk::kMbarSpin));
+    if (h->stream) VK_CUDA(h, cudaStreamSynchronize(h->stream));
+    drop_graph(h);                         // the captured loop has the old limit
+    h->spin = polls < 0 ? vk::kMbarSpin : polls;
     return VK_OK;
 }
 

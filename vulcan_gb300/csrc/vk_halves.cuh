@@ -23,13 +23,16 @@ __device__ __forceinline__ void cluster_sync_all() {
 }
 
 // The next of `units` from a counter, -1 when there is none left.  All threads
-// call it; in a cluster (CL) every CTA gets rank 0's.
+// call it; in a cluster (CL) every CTA gets rank 0's, -1 too once a CTA that gave
+// up a wait has set `lost` (NULL: none) in rank 0's shared memory: its word is
+// read between two cluster barriers, so all CTAs leave together.
 template <bool CL>
-__device__ __forceinline__ int next_unit(unsigned *queue, int units, int *s_unit, int rank, int csize) {
+__device__ __forceinline__ int next_unit(unsigned *queue, int units, int *s_unit, int rank, int csize,
+                                         const int *lost) {
     if (CL) {
         cluster_sync_all();
         if (rank == 0 && threadIdx.x == 0) {
-            const int u = (int)atomicAdd(queue, 1u);
+            const int u = lost && *(const volatile int *)lost ? units : (int)atomicAdd(queue, 1u);
             const uint32_t la = smem_u32(s_unit);
             for (int d = 0; d < csize; ++d)
                 asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(cluster_addr(la, (uint32_t)d)), "r"(u) : "memory");
@@ -44,19 +47,22 @@ __device__ __forceinline__ int next_unit(unsigned *queue, int units, int *s_unit
     return u < units ? u : -1;
 }
 template <bool CL>
-__device__ __forceinline__ int next_half(const DevBatch &b, int *s_unit, int rank, int csize) {
-    return next_unit<CL>(b.queue, 2 * b.ncols, s_unit, rank, csize);
+__device__ __forceinline__ int next_half(const DevBatch &b, int *s_unit, int rank, int csize,
+                                         const int *lost = nullptr) {
+    return next_unit<CL>(b.queue, 2 * b.ncols, s_unit, rank, csize, lost);
 }
 
 // True for the second of a column's halves to get here; what the first wrote
-// before is then visible.  All threads call it (in a cluster: of every CTA).
+// before is then visible.  All threads call it (in a cluster: of every CTA); a
+// cluster that lost a message (`lost` as in next_unit) does not count as there.
 template <bool CL>
-__device__ __forceinline__ bool second_half(const DevBatch &b, int c, int *s_unit, int rank, int csize) {
+__device__ __forceinline__ bool second_half(const DevBatch &b, int c, int *s_unit, int rank, int csize,
+                                            const int *lost = nullptr) {
     __threadfence();
     if (CL) {
         cluster_sync_all();
         if (rank == 0 && threadIdx.x == 0) {
-            const int a = (int)atomicAdd(b.queue + 1 + c, 1u);
+            const int a = lost && *(const volatile int *)lost ? -1 : (int)atomicAdd(b.queue + 1 + c, 1u);
             __threadfence();
             const uint32_t la = smem_u32(s_unit);
             for (int d = 0; d < csize; ++d)

@@ -132,6 +132,7 @@ struct DevBatch {
     int grid_rates[3];         // CTAs of k_rates with tiles of 1, 2 and 4 layers: all of
                                // them resident at once, each striding over the tiles
     int grid_prep;             // the same of k_prep32, over the layers (0: one CTA each)
+    int spin;                  // polls of a wait for another CTA's message before it gives up
 };
 
 // Grid of a per-layer kernel whose CTAs stride over the layers: as many CTAs

@@ -54,7 +54,8 @@ namespace {
 
 // This CTA's part of the shared memory at sm and of the blocks (rank of csize).
 template <bool CL>
-__device__ __forceinline__ Lu64Mem lu64_mem(double *sm, int n, int csize, int rank, int *s_sing, int *s_dead) {
+__device__ __forceinline__ Lu64Mem lu64_mem(double *sm, int n, int csize, int rank, int *s_sing, int *s_dead, int *s_lost,
+                                            int spin) {
     Lu64Mem m;
     m.n = n;
     m.csize = CL ? csize : 1;
@@ -77,6 +78,8 @@ __device__ __forceinline__ Lu64Mem lu64_mem(double *sm, int n, int csize, int ra
     m.kinv = m.perm + n;
     m.sing = s_sing;
     m.dead = s_dead;
+    m.lost = s_lost;
+    m.spin = spin;
     return m;
 }
 
@@ -169,7 +172,11 @@ __device__ __forceinline__ void lu64_half(const DevNet &net, const DevBatch &b, 
                 }
             }
             __syncthreads();
-            lu64_invert<CL>(m, phase);
+            if (!lu64_invert<CL>(m, phase)) {
+                // nothing of this block is stored; the cluster meets where it would have
+                if (!middle) second_half<CL>(b, c, s_unit, m.rank, m.csize, m.lost);
+                break;
+            }
             ++phase;
         }
         if (middle) {
@@ -181,13 +188,13 @@ __device__ __forceinline__ void lu64_half(const DevNet &net, const DevBatch &b, 
             break;
         }
         if (t == cnt) {
-            middle = second_half<CL>(b, c, s_unit, m.rank, m.csize);
+            middle = second_half<CL>(b, c, s_unit, m.rank, m.csize, CL ? m.lost : nullptr);
             if (!middle) break;
             for (int q = tid; q < n; q += nth) { m.rowid[q] = q; m.colid[q] = q; }
             __syncthreads();
         }
     }
-    if (tid == 0 && *m.dead) atomicExch(&status[c], VK_ETIMEOUT);
+    if (CL && tid == 0 && *m.dead) atomicExch(&status[c], VK_ETIMEOUT);
     else if (tid == 0 && m.rank == 0 && *m.sing)
         atomicCAS(&status[c], 0, *m.sing == 2 ? VK_ENAN : VK_ESINGULAR);
 }
@@ -199,6 +206,23 @@ __device__ __forceinline__ void lu64_open(const Lu64Mem &m) {
     cluster_sync_all();
 }
 
+// The cluster leaves: no message is on its way to a CTA that has left, or whose
+// memory has another use from here on.  A CTA that gave up waits, bounded, for
+// what was sent to it all the same: messages of the inversion it gave up in,
+// and of the next one from a CTA that had all of this one's.
+__device__ __forceinline__ void lu64_close(const Lu64Mem &m, unsigned phase) {
+    constexpr int kDrainPolls = 1 << 16;   // milliseconds; a message takes microseconds
+    if (*m.dead)
+        for (int k = threadIdx.x; k < m.n; k += blockDim.x) {
+            if (k >= m.c0 && k < m.c0 + m.w) continue;
+            if (!mbar_poll(&m.bar[k], phase & 1, kDrainPolls)) continue;
+            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;"
+                         ::"r"(smem_u32(&m.bar[k])), "r"((uint32_t)lu64_msg(m.n) * 8) : "memory");
+            mbar_poll(&m.bar[k], (phase + 1) & 1, kDrainPolls);
+        }
+    cluster_sync_all();
+}
+
 }  // namespace
 
 template <bool CL, bool DENSE>
@@ -207,14 +231,14 @@ k_lu64(DevNet net, DevBatch b, const double *__restrict__ jv, const double *__re
        const double *__restrict__ dB, const double *__restrict__ dC,
        const double *__restrict__ dt, double *G, int *status, int csize, int mid1) {
     extern __shared__ __align__(16) double sm[];
-    __shared__ int s_unit, s_sing, s_dead;
-    const Lu64Mem m = lu64_mem<CL>(sm, net.ni, csize, CL ? (int)cluster_rank() : 0, &s_sing, &s_dead);
-    if (threadIdx.x == 0) s_dead = 0;
+    __shared__ int s_unit, s_sing, s_dead, s_lost;
+    const Lu64Mem m = lu64_mem<CL>(sm, net.ni, csize, CL ? (int)cluster_rank() : 0, &s_sing, &s_dead, &s_lost, b.spin);
+    if (threadIdx.x == 0) s_dead = s_lost = 0;
     if (CL) lu64_open(m);
     unsigned phase = 0;
-    for (int u; (u = next_half<CL>(b, &s_unit, m.rank, m.csize)) >= 0;)
+    for (int u; (u = next_half<CL>(b, &s_unit, m.rank, m.csize, CL ? &s_lost : nullptr)) >= 0;)
         lu64_half<CL, DENSE>(net, b, m, jv, dA, dB, dC, dt, G, status, mid1, u, &s_unit, phase);
-    if (CL) cluster_sync_all();            // no message is still on its way to a CTA that has left
+    if (CL) lu64_close(m, phase);
 }
 
 // Clusters of two: the longest nlong half-columns are each shared by a
@@ -224,22 +248,23 @@ k_lu64_long(DevNet net, DevBatch b, const double *__restrict__ jv, const double 
             const double *__restrict__ dB, const double *__restrict__ dC,
             const double *__restrict__ dt, double *G, int *status) {
     extern __shared__ __align__(16) double sm[];
-    __shared__ int s_unit, s_sing, s_dead;
+    __shared__ int s_unit, s_sing, s_dead, s_lost;
     unsigned phase = 0;
-    if (threadIdx.x == 0) s_dead = 0;
+    if (threadIdx.x == 0) s_dead = s_lost = 0;
     {
-        const Lu64Mem m = lu64_mem<true>(sm, net.ni, 2, (int)cluster_rank(), &s_sing, &s_dead);
+        const Lu64Mem m = lu64_mem<true>(sm, net.ni, 2, (int)cluster_rank(), &s_sing, &s_dead, &s_lost, b.spin);
         lu64_open(m);
-        for (int u; (u = next_unit<true>(b.queue, b.nlong, &s_unit, m.rank, 2)) >= 0;)
+        for (int u; (u = next_unit<true>(b.queue, b.nlong, &s_unit, m.rank, 2, &s_lost)) >= 0;)
             lu64_half<true, false>(net, b, m, jv, dA, dB, dC, dt, G, status, -1, u, &s_unit, phase);
-        cluster_sync_all();
+        lu64_close(m, phase);
+        if (s_lost) return;                // the same in both CTAs: no wait follows next_unit
         // the barriers' memory holds data from here on
         for (int k = threadIdx.x; k < m.n; k += blockDim.x)
             asm volatile("mbarrier.inval.shared::cta.b64 [%0];" ::"r"(smem_u32(&m.bar[k])) : "memory");
         __syncthreads();
     }
-    const Lu64Mem m = lu64_mem<false>(sm, net.ni, 1, 0, &s_sing, &s_dead);
-    for (int u; (u = next_unit<false>(b.queue + 1 + b.ncols, 2 * b.ncols - b.nlong, &s_unit, 0, 1)) >= 0;)
+    const Lu64Mem m = lu64_mem<false>(sm, net.ni, 1, 0, &s_sing, &s_dead, &s_lost, 0);
+    for (int u; (u = next_unit<false>(b.queue + 1 + b.ncols, 2 * b.ncols - b.nlong, &s_unit, 0, 1, nullptr)) >= 0;)
         lu64_half<false, false>(net, b, m, jv, dA, dB, dC, dt, G, status, -1, b.nlong + u, &s_unit, phase);
 }
 
@@ -456,7 +481,9 @@ __host__ __device__ inline size_t sweep64c_smem(int n, int cs) {
 
 // sgn: sign of the couplings (+1: the solver's, A = D - dC - dB; -1: A = D + lower +
 // upper); gst: stride of the blocks; mid1: the middle layer, nz / 2 if negative;
-// a column whose status is not 0 is left alone if skip.
+// a column whose blocks were not inverted (status not 0) is left alone if skip -- all
+// but VK_ETIMEOUT, which another cluster may be writing here while this one's CTAs
+// read it, one before and one after.
 template <bool FWD>
 __global__ void __launch_bounds__(640)
 k_sweep64c(int n, int gst, DevBatch b, const double *G, const double *__restrict__ dB,
@@ -475,7 +502,8 @@ k_sweep64c(int n, int gst, DevBatch b, const double *G, const double *__restrict
     const bool rowt = row < r1, lead = rowt && part == 0;
     const int c = b.order[u >> 1], half = u & 1;
     // (the same for every CTA of the cluster)
-    if ((b.active && !b.active[c]) || (skip && status[c])) return;
+    const int st = skip ? *(volatile int *)&status[c] : 0;
+    if ((b.active && !b.active[c]) || (st != 0 && st != VK_ETIMEOUT)) return;
     const int l0 = b.col_off[c], nz = b.col_end[c] - l0, mid = mid1 >= 0 ? mid1 : nz / 2;
     const int nvis = half ? nz - 1 - mid : mid;
     const int first = FWD ? (half ? nz - 1 : 0) : (half ? mid + 1 : mid - 1);
@@ -521,13 +549,13 @@ k_sweep64c(int n, int gst, DevBatch b, const double *G, const double *__restrict
                 double x[12];
 #pragma unroll
                 for (int u = 0; u < 12; ++u) x[u] = 0.0;
-                for (int tries = 0;; ++tries) {
+                for (int tries = b.spin;; --tries) {
                     bool ok = true;
 #pragma unroll
                     for (int u = 0; u < 12; ++u)
                         if (q + 8 * u < n) ok &= get_tagged(xin + (uint32_t)(q + 8 * u) * 16u, x[u], tag);
                     if (ok) break;
-                    if ((tries & 255) == 255 && (tries >= kMbarSpin || *(volatile int *)&s_dead)) {
+                    if ((tries & 255) == 0 && (tries <= 0 || *(volatile int *)&s_dead)) {
                         *(volatile int *)&s_dead = 1;
                         break;
                     }
@@ -780,6 +808,7 @@ cudaError_t launch_solve64(int nz, int n, const double *D, const double *lo, con
     b.col_off = words + 1;
     b.col_end = words + 2;
     b.queue = reinterpret_cast<unsigned *>(words + 4);
+    b.spin = kMbarSpin;
     int *status = words + 3;
     k_solve64_words<<<1, 1, 0, s>>>(nz, words);
     const int cl = lu64_fits(n, 8) ? 8 : 1;

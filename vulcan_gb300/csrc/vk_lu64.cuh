@@ -66,15 +66,17 @@ __device__ __forceinline__ uint32_t cluster_rank() {
     asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
     return r;
 }
-// Bounded wait for data other CTAs of the cluster sent.
-__device__ __forceinline__ bool mbar_wait_cluster(uint64_t *bar, uint32_t parity) {
-    for (int i = 0; i < kMbarSpin; ++i) {
+// Wait of at most `spin` polls for data other CTAs of the cluster sent; false
+// when they run out or a CTA of the cluster has given up (*lost).
+__device__ __forceinline__ bool mbar_wait_cluster(uint64_t *bar, uint32_t parity, int spin, const int *lost) {
+    for (int i = 0; i < spin; ++i) {
         uint32_t ok;
         asm volatile("{\n\t.reg .pred p;\n\t"
                      "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
                      "selp.u32 %0, 1, 0, p;\n\t}"
                      : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
         if (ok) return true;
+        if ((i & 63) == 63 && *(const volatile int *)lost) return false;
     }
     return false;
 }
@@ -106,16 +108,31 @@ struct Lu64Mem {
     int *perm, *kinv;     // [n] pivot row of each step, step of each row
     uint64_t *bar;        // [n] message barriers (cluster)
     int *sing;            // first failure: 1 zero pivot, 2 no finite candidate
-    int *dead;            // a message never came: later waits return at once
+    int *dead;            // this CTA gave up a wait for a message (its own threads set it)
+    int *lost;            // a CTA of the cluster did (set from there)
     int n, w, c0;         // size, slice width, first column
     int csize, rank, pw;  // cluster size, rank, prep warps
+    int spin;             // polls of a wait
 };
+
+// A message never came: this CTA's block is void, and the others of the cluster,
+// which are all in the kernel until the cluster leaves it together, stop waiting.
+__device__ __forceinline__ void lu64_give_up(const Lu64Mem &m) {
+    if (*(volatile int *)m.dead) return;
+    *(volatile int *)m.dead = 1;
+    for (int c = 0; c < m.csize; ++c)
+        asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(cluster_addr(smem_u32(m.lost), (uint32_t)c)), "r"(1)
+                     : "memory");
+}
 
 // Inverts the block in m.S and relabels it.  All threads of the CTA call it
 // (in a cluster: of every CTA); it starts after a block barrier and ends with
-// one.  `phase`: inversions this CTA has done before (message parity).
+// one.  `phase`: inversions this CTA has done before (message parity).  False, for
+// the whole CTA, when a message never came: m.S then holds no inverse, rowid and colid
+// are as before, and no other inversion may follow (it would arm message
+// barriers whose phase is open, and relabel by pivots that never were).
 template <bool CL>
-__device__ __forceinline__ void lu64_invert(const Lu64Mem &m, unsigned phase) {
+__device__ __forceinline__ bool lu64_invert(const Lu64Mem &m, unsigned phase) {
     const int n = m.n, w = m.w, c0 = m.c0, c1 = c0 + w, ms = lu64_msg(n);
     const int tid = threadIdx.x, nth = blockDim.x, lane = tid & 31, warp = tid >> 5;
     const int npt = m.pw * 32;
@@ -198,9 +215,8 @@ __device__ __forceinline__ void lu64_invert(const Lu64Mem &m, unsigned phase) {
     const int i0 = tb >= 0 && w > 0 ? tb / w : 0, q0 = tb >= 0 && w > 0 ? tb - i0 * w : 0;
     for (int k = 0; k < n; ++k) {
         const double *slot = m.msg + (size_t)(CL ? k : (k & 1)) * ms;
-        if (CL && (k < c0 || k >= c1) && !*(volatile int *)m.dead) {
-            if (!mbar_wait_cluster(&m.bar[k], phase & 1)) *(volatile int *)m.dead = 1;
-        }
+        if (CL && (k < c0 || k >= c1))
+            if (!mbar_wait_cluster(&m.bar[k], phase & 1, m.spin, m.lost)) lu64_give_up(m);
         if (prep_thread) {
             if (mk != k) {                              // another CTA's step
                 mult = r < n ? slot[2 + r] : 0.0;
@@ -259,6 +275,7 @@ __device__ __forceinline__ void lu64_invert(const Lu64Mem &m, unsigned phase) {
         }
         __syncthreads();
     }
+    if (CL && *(volatile int *)m.dead) return false;    // (set before the last barrier only)
     // labels of the inverse
     int nr = 0, nc = 0;
     if (tid < n) {
@@ -271,6 +288,7 @@ __device__ __forceinline__ void lu64_invert(const Lu64Mem &m, unsigned phase) {
         m.colid[tid] = nc;
     }
     __syncthreads();
+    return true;
 }
 
 }  // namespace vk

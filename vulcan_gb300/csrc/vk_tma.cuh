@@ -10,7 +10,7 @@
 
 namespace vk {
 
-constexpr int kMbarSpin = 1 << 22;      // try_wait polls before giving up
+constexpr int kMbarSpin = 1 << 22;      // try_wait polls before giving up: 16 s (one that fails takes 7 760 cycles)
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) {
     return (uint32_t)__cvta_generic_to_shared(p);
@@ -39,6 +39,19 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, uint32_t parity) {
                  "selp.u32 %0, 1, 0, p;\n\t}"
                  : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
     return ok != 0;
+}
+
+// At most `polls` looks at phase `parity` of the barrier, none of which suspends.
+__device__ __forceinline__ bool mbar_poll(uint64_t *bar, uint32_t parity, int polls) {
+    for (int i = 0; i < polls; ++i) {
+        uint32_t ok;
+        asm volatile("{\n\t.reg .pred p;\n\t"
+                     "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+                     "selp.u32 %0, 1, 0, p;\n\t}"
+                     : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
+        if (ok) return true;
+    }
+    return false;
 }
 
 // Bounded wait for phase `parity` of the barrier; false on timeout.

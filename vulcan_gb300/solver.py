@@ -382,6 +382,10 @@ class Ros2Handle:
         (0: default) and, for capi.VK_TUNE_LU32, the register tiling (-1: by ni)."""
         check(lib().vk_set_launch(self.h, int(kernel), int(ctas_per_sm), int(variant)), self.h)
 
+    def set_wait_limit(self, polls=-1):
+        """Polls of a wait between the CTAs of the FP64 solve (vk_set_wait_limit; -1: built-in)."""
+        check(lib().vk_set_wait_limit(self.h, int(polls)), self.h)
+
     def get_launch(self, kernel):
         """(ctas_per_sm, variant) set for a kernel (vk_get_launch)."""
         c, v = C.c_int(), C.c_int()
