@@ -42,7 +42,7 @@ extern "C" {
 #define VK_ESINGULAR     3   /* zero pivot in a diagonal block */
 #define VK_ENAN          4   /* non-finite value in the state */
 #define VK_EMAXATTEMPT   5   /* attempt cap reached without an accepted step */
-#define VK_ETIMEOUT      6   /* host watchdog gave up waiting */
+#define VK_ETIMEOUT      6   /* the host watchdog, or a wait on the device, gave up */
 #define VK_ENOMEM        7   /* device allocation failed */
 
 /* ---- linear-solve precision ---- */

@@ -59,6 +59,25 @@ def test_a_message_that_never_comes(name, ncols):
     h.close()
 
 
+@pytest.mark.parametrize('precision', [capi.VK_PREC_FP64, capi.VK_PREC_MIXED])
+def test_an_attempt_reports_it(precision):
+    from vulcan_gb300.solver import ColumnBatch, GPUNetwork, Ros2Handle
+    net = Network.from_npz(os.path.join(GOLDEN, 'net_NCHO_thermo.npz'))
+    spec, it = _item(net, 'NCHO_thermo', 14)
+    b = ColumnBatch([it], net.ni)
+    h = Ros2Handle(GPUNetwork(net, spec.atom_list), 1, b.L, precision=precision)
+    h.set_columns(b)
+    h.set_route(1e-9)                            # mixed: this step is solved in FP64
+    ref = h.attempt(1e-8)
+    h.set_wait_limit(0)
+    with pytest.raises(capi.VkError) as e:
+        h.attempt(1e-8)
+    assert e.value.code == capi.VK_ETIMEOUT
+    h.set_wait_limit()
+    np.testing.assert_array_equal(h.attempt(1e-8)['sol'], ref['sol'])
+    h.close()
+
+
 def test_limit_is_checked():
     from vulcan_gb300.solver import GPUNetwork, Ros2Handle
     net = Network.from_npz(os.path.join(GOLDEN, 'net_CHO_thermo.npz'))

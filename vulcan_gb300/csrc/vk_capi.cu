@@ -753,6 +753,8 @@ extern "C" int vk_ros2_attempt(vk_handle *h, const double *dt, int flags, double
             return fail(h, VK_ESINGULAR, "singular diagonal block in column " + std::to_string(c));
         if (st[c] == VK_ENAN)
             return fail(h, VK_ENAN, "non-finite pivot (NaN state) in column " + std::to_string(c));
+        if (st[c] != VK_OK)
+            return fail(h, st[c], "a message or copy on the device never came, in column " + std::to_string(c));
     }
     return VK_OK;
 }
