@@ -252,6 +252,7 @@ int lu64_long(int n, int nsm, int clusters2, int ncols, const int *nz);
 void launch_lu64(const DevNet &net, const DevBatch &b, const Work &w, cudaStream_t s);
 // One column of given blocks (sizes and words: vk_lu64.cu).
 constexpr int kSolve64Words = 8;
+constexpr int kSolve64Grew = -1;         // status: from both ends it would lose digits
 cudaError_t init_solve64(int nmax);
 cudaError_t launch_solve64(int nz, int n, const double *D, const double *lo, const double *up, const double *rhs,
                            double *x, double *G, double *z, int *words, int mid, cudaStream_t s);

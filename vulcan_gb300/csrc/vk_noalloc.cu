@@ -16,8 +16,9 @@
 // two-sided block-Thomas (vk_lu64.cu): a cluster of eight CTAs per half of the
 // column.  A column of 150 layers of 69 species: 28.1 -> 3.7 ms (one CTA from
 // one end before).  Where the two-sided order meets a block without a finite
-// non-zero pivot, the column is solved once more from its bottom alone, whose
-// answer or failure is the call's.
+// non-zero pivot, or a Schur term from the top that would cost the block its
+// digits (k_solve64_growth), the column is solved from its bottom alone, whose answer or
+// failure is the call's (10.8 ms for such a column).
 #include <cuda_runtime.h>
 
 #include <cmath>
@@ -93,7 +94,8 @@ extern "C" int vk_block_solve_noalloc(int nz, int ni, const double *D, const dou
         return noalloc_fail(VK_ECUDA, std::string("CUDA error pending from earlier work (nothing launched): ") +
                                           cudaGetErrorString(e));
     int status = 0;
-    for (int mid = -1;; mid = nz - 1) {        // from both ends; from the bottom alone
+    // from both ends (of two layers the upper is the middle); from the bottom alone
+    for (int mid = nz < 3 ? nz - 1 : -1;; mid = nz - 1) {
         e = vk::launch_solve64(nz, ni, D, lower, upper, b, x, sc.p, sc.p + (size_t)nz * ni * ni, sc.words, mid, s);
         if (e == cudaSuccess) e = cudaGetLastError();
         if (e != cudaSuccess) return noalloc_fail(VK_ECUDA, std::string("launch: ") + cudaGetErrorString(e));
