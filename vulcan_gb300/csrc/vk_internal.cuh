@@ -254,6 +254,7 @@ void launch_lu64(const DevNet &net, const DevBatch &b, const Work &w, cudaStream
 constexpr int kSolve64Words = 8;
 constexpr int kSolve64Grew = -1;         // status: from both ends it would lose digits
 cudaError_t init_solve64(int nmax);
+bool solve64_small(int nz, int n);       // takes the bottom-up form, mid = nz - 1
 cudaError_t launch_solve64(int nz, int n, const double *D, const double *lo, const double *up, const double *rhs,
                            double *x, double *G, double *z, int *words, int mid, cudaStream_t s);
 void launch_fwd64(const DevNet &net, const DevBatch &b, const double *G, const double *dB,

@@ -812,6 +812,66 @@ k_solve64_growth(int nz, int n, const double *__restrict__ D, const double *__re
     }
 }
 
+// A small system in one launch: one CTA factorises from the bottom (words and G
+// stay its own) and does both sweeps, a warp per row.
+__global__ void __launch_bounds__(544)
+k_solve64_small(int nz, int n, const double *__restrict__ D, const double *__restrict__ lo,
+                const double *__restrict__ up, const double *rhs, double *x, double *G, double *z, int *words) {
+    extern __shared__ __align__(16) double sm[];
+    __shared__ int s_unit, s_sing, s_dead, s_lost;
+    const int tid = threadIdx.x, nth = blockDim.x, lane = tid & 31;
+    if (tid < kSolve64Words) words[tid] = tid == 2 ? nz : 0;    // order, col_off, col_end, status, queue
+    __syncthreads();
+    DevNet net = {};
+    net.ni = n;
+    DevBatch b = {};
+    b.ncols = 1;
+    b.order = words;
+    b.col_off = words + 1;
+    b.col_end = words + 2;
+    b.queue = reinterpret_cast<unsigned *>(words + 4);
+    const Lu64Mem m = lu64_mem<false>(sm, n, 1, 0, &s_sing, &s_dead, &s_lost, 0);
+    unsigned phase = 0;
+    for (int u = 0; u < 2; ++u) {          // the layers below the last one, the last one
+        lu64_half<false, true>(net, b, m, D, nullptr, up, lo, nullptr, G, words + 3, nz - 1, u, &s_unit, phase);
+        __syncthreads();
+    }
+    double *v = sm;                        // [n] the product's input
+    auto product = [&](int j, int r) {
+        const double *g = G + ((size_t)j * n + r) * n;
+        double s = 0.0;
+        for (int q = lane; q < n; q += 32) s = __fma_rn(g[q], v[q], s);
+        for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        return s;
+    };
+    const int warp = tid >> 5, nwarp = nth >> 5;
+    for (int j = 0; j < nz; ++j) {
+        const size_t e = (size_t)j * n;
+        for (int t = tid; t < n; t += nth) v[t] = j ? __fma_rn(-lo[e + t], z[e - n + t], rhs[e + t]) : rhs[t];
+        __syncthreads();
+        for (int r = warp; r < n; r += nwarp) {
+            const double s = product(j, r);
+            if (lane == 0) z[e + r] = s;
+        }
+        __syncthreads();
+    }
+    for (int j = nz - 1; j >= 0; --j) {
+        const size_t e = (size_t)j * n;
+        for (int t = tid; t < n && j + 1 < nz; t += nth) v[t] = -up[e + t] * x[e + n + t];
+        __syncthreads();
+        for (int r = warp; r < n; r += nwarp) {
+            const double s = j + 1 < nz ? product(j, r) : 0.0;
+            if (lane == 0) x[e + r] = z[e + r] + s;
+        }
+        __syncthreads();
+    }
+}
+// Where the four or five launches of the general form take longer than the layers
+// (us a call, this kernel and the general one: 1 layer of 1 species 26 and 37, 8 of 4 65
+// and 70, 3 of 16 65 and 70, 2 of 24 63 and 81; 12 of 4 88 and 82, 6 of 16 112 and 96, 3 of 24
+// 88 and 81).
+bool solve64_small(int nz, int n) { return n <= 32 && nz <= 8 && nz * n <= 48; }
+
 cudaError_t init_solve64(int nmax) {
     size_t scl = 0, ssc = 0;
     for (int n = 1; n <= nmax; ++n) {
@@ -822,12 +882,17 @@ cudaError_t init_solve64(int nmax) {
     if (e == cudaSuccess) e = raise_smem_limit(k_lu64<true, true>, scl);
     if (e == cudaSuccess) e = raise_smem_limit(k_sweep64c<true>, ssc);
     if (e == cudaSuccess) e = raise_smem_limit(k_sweep64c<false>, ssc);
+    if (e == cudaSuccess) e = raise_smem_limit(k_solve64_small, lu64_smem(nmax, 1));
     return e;
 }
 
 // G: nz n n doubles, z: nz n, words: kSolve64Words ints, words[3] the status.
 cudaError_t launch_solve64(int nz, int n, const double *D, const double *lo, const double *up, const double *rhs,
                            double *x, double *G, double *z, int *words, int mid, cudaStream_t s) {
+    if (mid == nz - 1 && solve64_small(nz, n)) {
+        k_solve64_small<<<1, lu64_threads(n, 1), lu64_smem(n, 1), s>>>(nz, n, D, lo, up, rhs, x, G, z, words);
+        return cudaGetLastError();
+    }
     DevNet net = {};
     net.ni = n;
     DevBatch b = {};

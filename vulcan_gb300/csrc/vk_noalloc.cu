@@ -94,8 +94,9 @@ extern "C" int vk_block_solve_noalloc(int nz, int ni, const double *D, const dou
         return noalloc_fail(VK_ECUDA, std::string("CUDA error pending from earlier work (nothing launched): ") +
                                           cudaGetErrorString(e));
     int status = 0;
-    // from both ends (of two layers the upper is the middle); from the bottom alone
-    for (int mid = nz < 3 ? nz - 1 : -1;; mid = nz - 1) {
+    // from both ends (of two layers the upper is the middle); from the bottom alone, as
+    // small systems are, in one launch
+    for (int mid = nz < 3 || vk::solve64_small(nz, ni) ? nz - 1 : -1;; mid = nz - 1) {
         e = vk::launch_solve64(nz, ni, D, lower, upper, b, x, sc.p, sc.p + (size_t)nz * ni * ni, sc.words, mid, s);
         if (e == cudaSuccess) e = cudaGetLastError();
         if (e != cudaSuccess) return noalloc_fail(VK_ECUDA, std::string("launch: ") + cudaGetErrorString(e));
