@@ -44,7 +44,6 @@ struct vk_handle {
     WDesc *d_w = nullptr;
     int *d_jptr = nullptr;
     int2 *d_jterm = nullptr;
-    int *d_jpos = nullptr;
     int *d_jrow = nullptr, *d_jcol = nullptr, *d_jrowptr = nullptr, *d_jmap = nullptr;
     double *d_compo = nullptr;
     int npc = 0;                        // pieces of the Jacobian rows (k_refine)
@@ -108,7 +107,7 @@ struct vk_handle {
         n.pairs = d_pairs; n.src_ptr = d_src_ptr; n.src = d_src; n.w = d_w;
         n.src_order = d_src_order; n.jorder = d_jorder;
         n.src_nu = d_src_nu; n.jterm_nu = d_jterm_nu;
-        n.jptr = d_jptr; n.jterm = d_jterm; n.jpos = d_jpos; n.compo = d_compo;
+        n.jptr = d_jptr; n.jterm = d_jterm; n.compo = d_compo;
         n.jrow = d_jrow; n.jcol = d_jcol; n.jrowptr = d_jrowptr; n.jmap = d_jmap;
         n.npc = npc; n.pc = d_pc; n.rpcptr = d_rpcptr; n.rpc = d_rpc;
         n.nxm = nxm; n.nh = nh; n.porder = d_porder; n.src_slot = d_src_slot; n.src_c = d_src_c;
@@ -281,7 +280,6 @@ extern "C" int vk_create(const vk_network *net, int max_cols, int max_layers, in
         TRY(upload(h, &h->d_jorder, order));
     }
     TRY(upload(h, &h->d_jterm, net->jterm));
-    TRY(upload(h, &h->d_jpos, net->jpos));
     TRY(upload(h, &h->d_compo, net->compo));
     TRY(upload(h, &h->d_jrow, net->jrow));
     TRY(upload(h, &h->d_jcol, net->jcol));

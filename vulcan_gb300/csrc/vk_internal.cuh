@@ -1,7 +1,6 @@
 // Internal declarations shared by the vk_* translation units.
 #pragma once
 
-#include <cuda.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <string>
@@ -83,7 +82,6 @@ struct DevNet {
     const int *jorder;         // [nnz] Jacobian entries by decreasing term count
     const int2 *jterm;
     const double *jterm_nu;
-    const int *jpos;
     const int *jrow, *jcol, *jrowptr, *jmap;
     // Jacobian rows cut into pieces of similar length (k_refine): piece i sums
     // entries [x, x + y); row s's pieces are rpc[rpcptr[s] .. rpcptr[s+1])
@@ -157,30 +155,6 @@ inline cudaError_t raise_smem_limit(K *kernel, size_t bytes) {
     if ((size_t)a.maxDynamicSharedSizeBytes >= bytes) return cudaSuccess;
     return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
-
-// Grid of a per-column kernel: CTAs per SM from vk_set_launch, else the
-// batch's override, else the kernel's default; never more than the columns.
-inline int column_grid(const DevBatch &b, int kernel, int cps_default) {
-    const int cps = b.cps_k[kernel] > 0 ? b.cps_k[kernel] : b.cps > 0 ? b.cps : cps_default;
-    const long long g = (long long)cps * b.nsm;
-    return (g > 0 && g < b.ncols) ? (int)g : b.ncols;
-}
-
-#ifdef __CUDACC__
-// Per-column kernels run as a work queue: each CTA takes the next column in
-// b.order (longest first) until the queue is empty, so the SMs finish
-// together however uneven the columns are.  All threads call it; returns -1
-// when no column is left.
-__device__ __forceinline__ int next_column(const DevBatch &b, int *s_col) {
-    __syncthreads();                 // everyone has read the previous s_col
-    if (threadIdx.x == 0) {
-        const unsigned i = atomicAdd(b.queue, 1u);
-        *s_col = i < (unsigned)b.ncols ? b.order[i] : -1;
-    }
-    __syncthreads();
-    return *s_col;
-}
-#endif
 
 // Photochemistry radiative transfer tables and state (vk_photo.cu).
 struct PhotoDev {

@@ -473,7 +473,7 @@ RefineShape refine_shape(int n, int npc, int nnz, int ctas) {
     RefineShape r;
     // lanes per product row, and a warp more for the copies
     const int rows = n <= 144 ? 288 : 320;
-    r.tpr = 4 * n <= rows ? 4 : 2 * n <= rows ? 2 : 1;
+    r.tpr = 4 * n <= rows ? 4 : 2;           // (2 VK_MAX_NI <= 320)
     r.nth = (r.tpr * n + 31) / 32 * 32 + 32;
     r.nb = 4;
     while (r.nb > 2 && ctas * ((size_t)refine_layout(n, npc, nnz, r.nth / 32, r.nb).end + 1200) > 233472) --r.nb;
@@ -484,8 +484,7 @@ RefineShape refine_shape(int n, int npc, int nnz, int ctas) {
 
 cudaError_t init_mixed_kernels(const DevNet &net) {
     const RefineShape r = refine_shape(net.ni, net.npc, net.nnz, 1);
-    return r.tpr == 4 ? raise_smem_limit(k_refine<4>, r.smem)
-         : r.tpr == 2 ? raise_smem_limit(k_refine<2>, r.smem) : raise_smem_limit(k_refine<1>, r.smem);
+    return r.tpr == 4 ? raise_smem_limit(k_refine<4>, r.smem) : raise_smem_limit(k_refine<2>, r.smem);
 }
 
 void launch_refine(const DevNet &net, const DevBatch &b, const Work &w, const double *rhs,
@@ -494,7 +493,7 @@ void launch_refine(const DevNet &net, const DevBatch &b, const Work &w, const do
     const RefineShape r = refine_shape(net.ni, net.npc, net.nnz, 2 * b.ncols <= b.nsm ? 1 : 2);
     reset_queue(b, s);
     const int grid = half_grid(b, VK_TUNE_REFINE, 2) & ~1;    // CTA pairs, one column each
-    auto kernel = r.tpr == 4 ? k_refine<4> : r.tpr == 2 ? k_refine<2> : k_refine<1>;
+    auto kernel = r.tpr == 4 ? k_refine<4> : k_refine<2>;
     kernel<<<grid, r.nth, r.smem, s>>>(net, b, w.G32, w.rs, w.cs, w.jv, w.dA, w.dB, w.dC, w.dt,
                                       rhs, x, w.zf, w.wcf, w.wcb, w.raf, w.xf, yscale, yk2, w.y,
                                       max_sweeps, tol,

@@ -1,6 +1,5 @@
 // Preparation of the mixed path's FP32 factorisation (vk_lu32.cu): per layer the
 // scales R_j, S_j and the dense scaled block R_j D_j S_j.
-#include <cuda.h>
 #include <cuda_runtime.h>
 #include <math.h>
 
