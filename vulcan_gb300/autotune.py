@@ -2,7 +2,7 @@
 
 The work-queue kernels (the FP32 and FP64 block-Thomas factorisations, the
 FP64 sweeps and the mixed-precision refinement) run ``ctas_per_sm`` CTAs per
-SM, and the FP32 Gauss-Jordan keeps its block in one of four register
+SM, and the FP32 Gauss-Jordan keeps its block in one of six register
 tilings.  Which choice fills the SMs best depends on the species count, the
 batch's number of columns and spread of nz, the precision path and the GPU.
 ``tune`` measures candidate settings on the caller's own batch -- one Ros2
@@ -30,6 +30,7 @@ KERNELS = {
     'sweep64': (capi.VK_TUNE_SWEEP64, (capi.VK_PREC_FP64, capi.VK_PREC_MIXED)),
 }
 CTAS_PER_SM = (1, 2, 3, 4)
+LU32_TILES = (48, 64, 72, 96, 128, 160)    # species the register tilings of k_lu32 cover
 
 
 def candidates(kernel, ni, ctas=CTAS_PER_SM):
@@ -39,6 +40,13 @@ def candidates(kernel, ni, ctas=CTAS_PER_SM):
         tilings = [t for t, cap in enumerate(capi.LU32_TILING_CAP) if cap >= ni]
         return [(c, t) for t in tilings for c in ctas]
     return [(c, -1) for c in ctas]
+
+
+def lu32_tile(ni, variant):
+    """The register tiling (species it covers) that an LU32 variant launches for
+    ni species: several variants may name the same one."""
+    want = max(ni, capi.LU32_TILING_CAP[variant]) if 0 <= variant < 4 else ni
+    return next(t for t in LU32_TILES if t >= want)
 
 
 def attempt_ms(h, dt, flags, repeats=3):
@@ -69,7 +77,12 @@ def tune(h, dt, flags=capi.VK_F_MOLDIFF, precision=capi.VK_PREC_MIXED, ni=None,
     for _ in range(passes):
         for k in names:
             kid = KERNELS[k][0]
+            seen = set()
             for c, v in candidates(k, ni):
+                same = (c, lu32_tile(ni, v) if k == 'lu32' else v)
+                if same in seen:             # launches what was measured already
+                    continue
+                seen.add(same)
                 h.set_launch(kid, c, v)
                 ms = attempt_ms(h, dt, flags, repeats)
                 if log is not None:
