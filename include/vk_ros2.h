@@ -293,9 +293,13 @@ VK_API int  vk_set_rate_caps(vk_handle *h, const int *kind, const double *t_max,
                              const double *params);
 VK_API int  vk_compute_k(vk_handle *h);
 /* ---- launch tuning (for an autotuner; no counterpart in the reference) ----
- * The per-column kernels take columns from a work queue; their grid is
- * ctas_per_sm x SMs CTAs.  kernel: VK_TUNE_*; ctas_per_sm 0..8 (0: the
- * kernel's built-in default, or VK_CTAS_PER_SM from the environment);
+ * The per-column kernels take half-columns (k_refine: columns) from a work
+ * queue; their grid is ctas_per_sm x SMs CTAs, at most one per half-column.
+ * kernel: VK_TUNE_*; ctas_per_sm 0..8 (0: the kernel's built-in default, or
+ * VK_CTAS_PER_SM from the environment).  Where every half-column can have an
+ * SM to itself, VK_TUNE_LU64 shares the blocks (or those of the longest halves)
+ * between the CTAs of clusters whatever is set, and so does VK_TUNE_SWEEP64
+ * where each can have two.
  * variant: for VK_TUNE_LU32 the register tiling of the FP32 Gauss-Jordan:
  * 0..3 at least the one for blocks of 48, 80, 112, 160 species, 4 and 5 (up
  * to 128 species) and -1 the smallest that holds ni; a variant smaller than

@@ -78,6 +78,29 @@ def test_an_attempt_reports_it(precision):
     h.close()
 
 
+@pytest.mark.parametrize('ncols', [1, 50])
+def test_ctas_per_sm_leave_the_sharing_as_it_is(ncols):
+    """A number of CTAs per SM (a tuning file's, say) does not take from the long halves
+    of a batch the CTAs they share: with no polls allowed it fails like the default."""
+    from vulcan_gb300.solver import ColumnBatch, GPUNetwork, Ros2Handle
+    net = Network.from_npz(os.path.join(GOLDEN, 'net_NCHO_thermo.npz'))
+    items = [_item(net, 'NCHO_thermo', nz, seed=nz) for nz in (9, 14, 21)]
+    b = ColumnBatch([items[c % 3][1] for c in range(ncols)], net.ni)
+    h = Ros2Handle(GPUNetwork(net, items[0][0].atom_list), ncols, b.L)
+    h.set_columns(b)
+    ref = h.attempt(1e-8)
+    for ctas in (1, 2, 4):
+        h.set_launch(capi.VK_TUNE_LU64, ctas)
+        h.set_launch(capi.VK_TUNE_SWEEP64, ctas)
+        np.testing.assert_array_equal(h.attempt(1e-8)['sol'], ref['sol'])
+        h.set_wait_limit(0)
+        with pytest.raises(capi.VkError) as e:
+            h.attempt(1e-8)
+        assert e.value.code == capi.VK_ETIMEOUT
+        h.set_wait_limit()
+    h.close()
+
+
 def test_limit_is_checked():
     from vulcan_gb300.solver import GPUNetwork, Ros2Handle
     net = Network.from_npz(os.path.join(GOLDEN, 'net_CHO_thermo.npz'))

@@ -730,7 +730,8 @@ int lu64_long(int n, int nsm, int clusters2, int ncols, const int *nz) {
 void launch_lu64(const DevNet &net, const DevBatch &b, const Work &w, cudaStream_t s) {
     const int n = net.ni, cs = cluster_size(b, b.ncl_lu, lu64_fits, n);
     reset_queue(b, s);
-    if (b.nlong > 0 && cs == 1 && b.cps == 0 && b.cps_k[VK_TUNE_LU64] == 0) {
+    // (whatever CTAs per SM are set: lu64_long shares halves only where each has an SM to itself)
+    if (b.nlong > 0 && cs == 1) {
         const ClusterLaunch L(std::min(b.ncl_lu[0], b.nsm / 2) * 2, lu64_threads(n, 1),
                               std::max(lu64_smem(n, 1), lu64_smem(n, 2)), 1, s);
         cudaLaunchKernelEx(&L.cfg, k_lu64_long, net, b, (const double *)w.jv, (const double *)w.dA,
