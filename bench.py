@@ -400,7 +400,8 @@ def run_gpu(args):
     roof['frac'] = roof['achieved'] / roof['peak']
     # DRAM bytes per launch: the ncu capture's bytes per layer (captured on the
     # 69-species workload) x this launch's layers; none for other networks
-    tpl, tsrc = profile_traffic(roof['kernel'].split()[0]) if args.workload == 'c2' else (None, None)
+    captured = {'k_lu32': 'k_lu32<3,18,4>', 'k_refine': 'k_refine'}[roof['kernel'].split()[0]]
+    tpl, tsrc = profile_traffic(captured) if args.workload == 'c2' else (None, None)
     roof['traffic'] = round(tpl * L) if tpl else None
     if tpl:
         roof['traffic_source'] = ('ncu capture summarised in %s: DRAM bytes per layer x the '

@@ -415,8 +415,9 @@ VK_API int  vk_chem_source(vk_handle *h, const double *y, double *dydt);
  * state and its last attempt untouched. */
 VK_API int  vk_rhs(vk_handle *h, const double *y, int flags, double *f);
 /* FP32 inverses of the scaled diagonal blocks of the last mixed-precision
- * attempt, [L][ni*ni] row-major (columns that attempt solved in FP64 hold
- * stale values). */
+ * attempt, less the Schur term of the layer below in a column's lower half, of
+ * the layer above in its upper half and of both in layer nz / 2; [L][ni*ni]
+ * row-major (columns that attempt solved in FP64 hold stale values). */
 VK_API int  vk_get_lu32(vk_handle *h, float *G);
 /* LHS pieces of the last attempt: -J entries [L][nnz_jac] in the order of
  * vk_network_jac_pattern, and the transport coefficients dA/dB/dC [L][ni]
