@@ -7,6 +7,7 @@
 #include <cstring>
 #include <new>
 #include <string>
+#include <unordered_map>
 #include <vector>
 
 #include <chrono>
@@ -908,15 +909,17 @@ static void rate_table(int npair, const int *kind, const double *params, std::ve
                        std::vector<int> &tab_off, std::vector<double> &val, std::vector<int4> &idx,
                        std::vector<int> &special) {
     std::vector<double> B, C;              // of the open chunk
+    std::unordered_map<unsigned long long, int> atB, atC;       // their entries by the value's bits
     int sp[7] = {};
     idx.assign(npair, make_int4(0, 0, 0, 0));
     pair_off.assign(1, 0);
     tab_off.assign(1, 0);
-    auto find = [](std::vector<double> &v, double x) {
-        size_t i = 0;
-        while (i < v.size() && std::memcmp(&v[i], &x, sizeof x) != 0) ++i;
-        if (i == v.size()) v.push_back(x);
-        return (int)i;
+    auto find = [&](std::vector<double> &v, double x) {
+        unsigned long long bits;
+        std::memcpy(&bits, &x, sizeof x);
+        const auto r = (&v == &B ? atB : atC).emplace(bits, (int)v.size());
+        if (r.second) v.push_back(x);
+        return r.first->second;
     };
     auto close = [&](int p) {
         const int nB = (int)B.size();      // C's entries follow B's
@@ -929,6 +932,8 @@ static void rate_table(int npair, const int *kind, const double *params, std::ve
         pair_off.push_back(p);
         B.clear();
         C.clear();
+        atB.clear();
+        atC.clear();
         std::fill(sp, sp + 7, 0);
     };
     for (int p = 0; p < npair; ++p) {
