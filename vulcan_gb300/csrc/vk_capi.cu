@@ -1094,6 +1094,12 @@ extern "C" int vk_photo_setup(vk_handle *h, int nbins, const double *bins, const
         topv(sflux_top, sflux_top + nbins), scv;
     std::vector<int> asv(abs_sp, abs_sp + nabs), apv(abs_photo, abs_photo + nabs),
         kiv(ch_kindex, ch_kindex + nch), ssv;
+    // channels of one rate: the last one's J is the rate (the kernel writes them side by side)
+    std::vector<char> taken((size_t)h->nr + 1, 0);
+    for (int c = nch - 1; c >= 0; --c) {
+        if (taken[kiv[c]]) kiv[c] = 0;
+        else taken[kiv[c]] = 1;
+    }
     if (nscat) {
         scv.assign(cross_scat, cross_scat + (size_t)nscat * nbins);
         ssv.assign(scat_sp, scat_sp + nscat);

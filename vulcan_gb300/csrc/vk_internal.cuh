@@ -166,7 +166,7 @@ struct PhotoDev {
     const double *cross_scat;  // [nscat][nbins] Rayleigh cross sections
     const int *scat_sp;        // [nscat]
     const double *wcross_J;    // [nch][nbins] photolysis cross section x J bin weight
-    const int *ch_kindex;      // [nch] 1-based k index of the channel
+    const int *ch_kindex;      // [nch] 1-based k index of the channel (0: a later channel has it)
     const double *sflux_top;   // [nbins] top-of-atmosphere flux
     double sl_angle, edd, f_diurnal, flux_atol;
     double *tau, *dflux_u, *dflux_d;   // [(L + ncols)][nbins] staggered

@@ -315,7 +315,8 @@ k_photo_J(DevNet net, DevBatch b, PhotoDev ph, double *k, unsigned long long *ch
             const int ch = ch0 + g + x * G;
             if (c >= 0 && ch < ph.nch) {
                 ph.J[l * ph.nch + ch] = acc[x];
-                k[l * net.nr + ph.ch_kindex[ch] - 1] = acc[x] * ph.f_diurnal;
+                const int ki = ph.ch_kindex[ch];
+                if (ki > 0) k[l * net.nr + ki - 1] = acc[x] * ph.f_diurnal;
             }
         }
     }
